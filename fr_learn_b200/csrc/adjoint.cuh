@@ -52,7 +52,7 @@ struct AdjArgs {
   double *trY;            // traces of Y [NV][NF][nE] (face kernel out)
   double *fnbar;          // this element's common-flux adjoint [NV][NF][nE] (face kernel out)
   const int *nbr;         // [NF][nE]
-  const double *nrm, *dA, *JG, *detJ;
+  const double *nrm, *dA, *JG, *detJ, *invDet;
   int vcjh;
   unsigned *err;
   // outputs of the element kernel

@@ -6,6 +6,7 @@
 #include "adjoint.cuh"
 #include "adjoint_visc.cuh"
 #include "dispatch.h"
+#include "kernels_line.cuh"
 #include "optab_upload.cuh"
 
 namespace frg {
@@ -36,11 +37,20 @@ void launch_wallp(const double *U, const int *nbr, const double *dA, const doubl
   fr_obj_wallp_kernel<C><<<(nE + 127) / 128, 128, 0, st>>>(U, nbr, dA, wsurf, vcjh, nE, L, bcWall, ph, grad, part);
 }
 
-// Viscous residuals: the forward gradient / projected-flux pass (the
-// generic gradient kernel on the stage state), then the two adjoint passes.
+// Block of the forward gradient pass: a narrow tile (the adjoint's meshes are
+// small) with as many lines in flight as fit.
+template <class C>
+struct AdjGradShape {
+  static constexpr int TE = C::DIM == 2 ? 16 : C::P < 3 ? 8 : 4;
+  static constexpr int L = (C::DIM == 2 ? 2 * C::N1 : 3 * C::N1 * C::N1) * TE;
+  static constexpr int NT = ((L + 31) & ~31) < 320 ? (L + 31) & ~31 : 320;
+  using T = LineT<C, double, TE, NT>;
+};
+// Viscous residuals: the forward gradient / projected-flux pass on the stage
+// state, then the two adjoint passes.
 template <class C, bool BC, int RS>
 void launch_adjv_elem(const AdjArgs &a, cudaStream_t st) {
-  using TV = TileV<C, double>;
+  using TV = AdjGradShape<C>;
   StageArgs f{};
   f.nE = a.nE;
   f.nEle = a.nEle;
@@ -51,7 +61,7 @@ void launch_adjv_elem(const AdjArgs &a, cudaStream_t st) {
   f.nrm = a.nrm;
   f.dA = a.dA;
   f.JG = a.JG;
-  f.detJ = a.detJ;
+  f.invDet = a.invDet;
   f.err = a.err;
   f.vcjh = a.vcjh;
   f.flags = SF_RESIDUAL;
@@ -68,7 +78,8 @@ void launch_adjv_elem(const AdjArgs &a, cudaStream_t st) {
     return t;
   }();
   set_stage_ops(f, ops[a.vcjh]);
-  fr_visc_grad_kernel<C, double, double, BC><<<(a.nEle + TV::TE - 1) / TV::TE, C::NT, TV::SMEM, st>>>(f);
+  fr_line_grad_kernel<C, double, double, BC, TV::TE, TV::NT, 1>
+      <<<(a.nEle + TV::TE - 1) / TV::TE, TV::NT, TV::T::SMEM, st>>>(f);
   using T = AdjViscTile<C>;
   fr_adjv_elem_kernel<C, BC, RS><<<(a.nEle + T::TE - 1) / T::TE, T::NT, T::SMEM, st>>>(a);
   fr_adjv_out_kernel<C, BC><<<(a.nEle + 3) / 4, 128, 0, st>>>(a);
@@ -77,7 +88,7 @@ void launch_adjv_elem(const AdjArgs &a, cudaStream_t st) {
 template <class C, bool BC, int RS>
 bool make_adjv(AdjSet &k, std::string &err) {
   using T = AdjViscTile<C>;
-  using TV = TileV<C, double>;
+  using TV = AdjGradShape<C>;
   k.face = &launch_adj_face<C>;
   k.elem = &launch_adjv_elem<C, BC, RS>;
   k.TE = T::TE;
@@ -90,8 +101,8 @@ bool make_adjv(AdjSet &k, std::string &err) {
   cudaError_t e = cudaFuncSetAttribute(fr_adjv_elem_kernel<C, BC, RS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)T::SMEM);
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(fr_visc_grad_kernel<C, double, double, BC>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TV::SMEM);
+    e = cudaFuncSetAttribute(fr_line_grad_kernel<C, double, double, BC, TV::TE, TV::NT, 1>,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TV::T::SMEM);
   if (e != cudaSuccess) { err = std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e); return false; }
   return true;
 }

@@ -15,9 +15,6 @@
 namespace frg {
 
 struct KernelSet {
-  void (*stage)(const void *args, int nBlk, size_t smem, cudaStream_t st) = nullptr;
-  // viscous configurations: the gradient kernel launched before each stage
-  void (*grad)(const void *args, int nBlk, size_t smem, cudaStream_t st) = nullptr;
   // traces of a double state: nE is the element stride of the trace array,
   // nEle the number of real elements, ldU the element stride of U
   void (*trace)(const double *U, void *tr, int nE, int nEle, int ldU, int vcjh, cudaStream_t st) = nullptr;
@@ -37,20 +34,18 @@ struct KernelSet {
   static constexpr int kMaxTma = 16;
   TmaVariant tma[kMaxTma];
   int nTma = 0;
-  int TE = 0;       // elements per block
-  int NT = 0;       // threads per block
-  size_t smem = 0;  // dynamic shared memory per block
-  // 3D viscous configurations: the fused update's two passes with TMA tile
-  // movement (gradient / projected viscous flux, then the stage); `maps`
-  // points at a ViscMaps built for tiles of vTE elements
-  void (*vgrad)(const void *args, const void *maps, int nBlk, size_t smem, cudaStream_t st) = nullptr;
-  void (*vstage)(const void *args, const void *maps, int nBlk, size_t smem, cudaStream_t st) = nullptr;
-  int vTE = 0;
-  int vPadG = 0;  // points per padding slot of their tiles' point layout
-  // resident blocks per SM of the two passes (their grids are persistent:
-  // at most SMs x this many blocks, each walking tiles)
-  int vgradOcc = 0, vstageOcc = 0;
-  size_t vgradSmem = 0, vstageSmem = 0;
+  // the line kernels (kernels_line.cuh) by block shape, widest tile first; grad: the viscous
+  // configurations' first pass, launched before each stage
+  struct LineVariant {
+    void (*stage)(const void *args, int nBlk, size_t smem, cudaStream_t st) = nullptr;
+    void (*grad)(const void *args, int nBlk, size_t smem, cudaStream_t st) = nullptr;
+    int TE = 0;
+    int rounds = 0;  // of the line-wise phases
+    size_t smem = 0;
+  };
+  static constexpr int kMaxLine = 3;
+  LineVariant line[kMaxLine];
+  int nLine = 0;
 };
 
 struct KernelKey {

@@ -19,7 +19,6 @@
 #include "dispatch.h"
 #include "kernels.cuh"
 #include "kernels_tma.cuh"
-#include "kernels_visc_tma.cuh"
 #include "adjoint.cuh"
 #include "setup.h"
 
@@ -207,7 +206,8 @@ struct frg_solver {
   HostGeom g;
   Ops1D ops;
   KernelSet ks;
-  int nV = 0, nS = 0, nF = 0, nE = 0, nBlk = 0, nRK = 0;
+  const KernelSet::LineVariant *line = nullptr;  // block shape of the line kernels for this mesh
+  int nV = 0, nS = 0, nF = 0, nE = 0, nBlk = 0, nRK = 0;  // nBlk: line kernels' blocks
   int L = 0;  // element stride of device arrays: nE rounded up to a multiple of 32
   size_t sstore = 8;  // bytes of the stored type
   std::vector<double> RKa, RKb;
@@ -247,18 +247,12 @@ struct frg_solver {
   bool dtFresh = false;  // device dt was computed from the current wave speeds
   // tensor maps of the TMA stage kernel
   bool useTma = false;
-  bool pdl = true;  // programmatic dependent launch between TMA stages (FRG_PDL=0: off)
+  bool pdl = true;  // programmatic dependent launch between stages (FRG_PDL=0: off)
   bool useGraph = true;  // steps replayed from captured graphs (FRG_GRAPH=0: launched directly)
   int nSM = 0;      // multiprocessors of the device (persistent grids)
   int tmaVar = 0;  // tile-shape variant of the TMA kernel (frg_autotune)
   int nBlkTma = 0;
   CUtensorMap mU, mAcc, mW[2], mTr[2], mJG, mDet, mNrm, mDA, mNbr;
-  // tensor maps of the 3D viscous TMA passes (tiles of ks.vTE elements):
-  // stage inputs W[i] in the padded point layout, and the rest
-  bool useViscTma = false;
-  struct {
-    CUtensorMap Win[2], U, Acc, Wout[2], tr[2], JG, det, nrm, dA, nbr, fvn, fvn2;
-  } vm;
   AdjState *adj = nullptr;
   // frg_apply_operator: operator images for the tensor-core GEMM, [which][dim]
   float *opImg[5][3] = {};
@@ -404,7 +398,7 @@ StageArgs base_args(frg_solver *s) {
   a.nrm = s->nrm;
   a.dA = s->dAs;
   a.JG = s->JG;
-  a.detJ = s->detJs;
+  a.invDet = s->invDetS;
   a.waveSp = s->waveSp;
   a.dt = s->p.dtType == 2 ? s->eleDt : dt_slot(s, s->dtCur);
   a.grp = s->grp;
@@ -465,72 +459,6 @@ frg_status make_map(CUtensorMap *m, void *base, CUtensorMapDataType dt, int esz,
   return FRG_OK;
 }
 
-// Tensor map of `rank` dimensions: dims in elements (innermost first),
-// strides in bytes of dimensions 1..rank-1, box extents.
-frg_status make_map_nd(CUtensorMap *m, void *base, CUtensorMapDataType dt, int esz, int rank, const cuuint64_t *dims,
-                       const cuuint64_t *strides, const cuuint32_t *box) {
-  EncodeTiledFn enc = encode_fn();
-  if (!enc) return fail(FRG_ERR_CUDA, "cuTensorMapEncodeTiled unavailable");
-  if (((size_t)box[0] * esz) % 16 || ((uintptr_t)base & 15)) return fail(FRG_ERR_ARG, "tensor map not TMA-compatible");
-  for (int i = 0; i < rank; i++)
-    if (box[i] < 1 || box[i] > 256) return fail(FRG_ERR_ARG, "tensor map box extent out of range");
-  for (int i = 0; i < rank - 1; i++)
-    if (strides[i] % 16) return fail(FRG_ERR_ARG, "tensor map stride not a multiple of 16 bytes");
-  cuuint32_t es[5] = {1, 1, 1, 1, 1};
-  CUresult r = enc(m, dt, (cuuint32_t)rank, base, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                   CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) return fail(FRG_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r);
-  return FRG_OK;
-}
-
-// Maps of the 3D viscous TMA passes (kernels_visc_tma.cuh, ViscMaps).
-frg_status setup_visc_tma(frg_solver *s) {
-  const int TE = s->ks.vTE, d = s->p.nDims, n1 = s->p.order + 1, nS = s->nS, nF = s->nF, nV = s->nV;
-  const cuuint64_t L = (cuuint64_t)s->L;
-  const int es = (int)s->sstore;
-  const CUtensorMapDataType ts = es == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
-  const cuuint32_t te = (cuuint32_t)TE;
-  auto map3 = [&](CUtensorMap *m, void *base, CUtensorMapDataType dt, int esz, int rows, int planes) {
-    const cuuint64_t dims[3] = {L, (cuuint64_t)rows, (cuuint64_t)planes};
-    const cuuint64_t str[2] = {L * esz, L * esz * rows};
-    const cuuint32_t box[3] = {te, (cuuint32_t)rows, (cuuint32_t)planes};
-    return make_map_nd(m, base, dt, esz, 3, dims, str, box);
-  };
-  auto map2 = [&](CUtensorMap *m, void *base, CUtensorMapDataType dt, int esz, int rows) {
-    const cuuint64_t dims[2] = {L, (cuuint64_t)rows};
-    const cuuint64_t str[1] = {L * esz};
-    const cuuint32_t box[2] = {te, (cuuint32_t)rows};
-    return make_map_nd(m, base, dt, esz, 2, dims, str, box);
-  };
-  // stage input in the padded point layout: each group of pg points walked
-  // with a box one point wider (the extra point is outside the tensor: zeros)
-  const int pg = s->ks.vPadG;
-  (void)n1;
-  auto map_padded = [&](CUtensorMap *m, void *base) {
-    const cuuint64_t dims[4] = {L, (cuuint64_t)pg, (cuuint64_t)(nS / pg), (cuuint64_t)nV};
-    const cuuint64_t str[3] = {L * es, L * es * pg, L * es * nS};
-    const cuuint32_t box[4] = {te, (cuuint32_t)(pg + 1), (cuuint32_t)(nS / pg), (cuuint32_t)nV};
-    return make_map_nd(m, base, ts, es, 4, dims, str, box);
-  };
-  const CUtensorMapDataType f64 = CU_TENSOR_MAP_DATA_TYPE_FLOAT64;
-  frg_status st;
-  if ((st = map_padded(&s->vm.Win[0], s->W[0])) || (st = map_padded(&s->vm.Win[1], s->W[1])) ||
-      (st = map3(&s->vm.U, s->U, f64, 8, nS, nV)) || (st = map3(&s->vm.Acc, s->Acc, f64, 8, nS, nV)) ||
-      (st = map3(&s->vm.Wout[0], s->W[0], ts, es, nS, nV)) || (st = map3(&s->vm.Wout[1], s->W[1], ts, es, nS, nV)) ||
-      (st = map3(&s->vm.tr[0], s->tr[0], ts, es, nF, nV)) || (st = map3(&s->vm.tr[1], s->tr[1], ts, es, nF, nV)) ||
-      (st = map3(&s->vm.JG, s->JG, ts, es, nS, d * d)) || (st = map2(&s->vm.det, s->invDetS, ts, es, nS)) ||
-      (st = map3(&s->vm.nrm, s->nrm, ts, es, nF, d)) || (st = map2(&s->vm.dA, s->dAs, ts, es, nF)) ||
-      (st = map3(&s->vm.fvn, s->fvn, ts, es, nF, nV)) ||
-      (st = map3(&s->vm.fvn2, s->visc2 ? s->fvn2 : s->fvn, ts, es, nF, nV)))
-    return st;
-  if (TE * 4 >= 16) {
-    if ((st = map2(&s->vm.nbr, s->nbr, CU_TENSOR_MAP_DATA_TYPE_INT32, 4, nF))) return st;
-  } else {
-    s->vm.nbr = s->vm.det;  // codes read by plain loads; the map is not used
-  }
-  return FRG_OK;
-}
-
 frg_status setup_tma(frg_solver *s) {
   const int TE = s->ks.tma[s->tmaVar].TE, L = s->L, d = s->p.nDims;
   const CUtensorMapDataType ts = s->sstore == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
@@ -560,13 +488,28 @@ frg_status setup_tma(frg_solver *s) {
   return FRG_OK;
 }
 
+// The line kernels' block shape for this mesh: the first that still gives every
+// other SM a block, or, where a block takes its lines in rounds, four blocks to
+// three SMs (both sides measured, see line_shape: a half-full GPU of wide tiles
+// is as fast as a full one of tiles half as wide, a quarter-full one is not).
+void pick_line(frg_solver *s) {
+  for (int i = 0; i < s->ks.nLine; i++) {
+    s->line = &s->ks.line[i];
+    s->nBlk = (s->nE + s->line->TE - 1) / s->line->TE;
+    if (s->line->rounds > 1 ? 3 * s->nBlk >= 4 * s->nSM : 2 * s->nBlk >= s->nSM) return;
+  }
+}
+
 frg_status launch_stage_args(frg_solver *s, StageArgs &a) {
-  if (s->ks.grad) {  // viscous: the gradient kernel first (same inputs)
-    s->ks.grad(&a, s->nBlk, s->ks.smem, s->stream);
+  const int flags = a.flags;
+  if (s->line->grad) {  // viscous: the gradient pass first (same inputs)
+    s->line->grad(&a, s->nBlk, s->line->smem, s->stream);
     frg_status st = post_launch(s);
     if (st) return st;
+    if (s->pdl) a.flags |= SF_PDL;  // the stage follows its gradient pass
   }
-  s->ks.stage(&a, s->nBlk, s->ks.smem, s->stream);
+  s->line->stage(&a, s->nBlk, s->line->smem, s->stream);
+  a.flags = flags;
   return post_launch(s);
 }
 
@@ -599,8 +542,8 @@ void drop_graphs(frg_solver *s) {
   s->graphEpoch++;
 }
 
-// The last stage of the TMA kernel computes the next step's global CFL dt.
-bool fused_dt(const frg_solver *s) { return s->useTma && s->p.dtType == 1; }
+// The last stage of a fused step computes the next step's global CFL dt.
+bool fused_dt(const frg_solver *s) { return s->p.dtType == 1; }
 
 frg_status launch_group_step(frg_solver *s) {
   fr_group_step_kernel<<<(s->nGrp + 127) / 128, 128, 0, s->stream>>>(
@@ -649,7 +592,6 @@ frg_status enqueue_step(frg_solver *s, int mode, cudaEvent_t *ev = nullptr) {
     a.aNext = jam ? s->RKa[k + 1] : (last ? 0.0 : s->RKa[k + 1]);
     a.bCur = jam ? 0.0 : s->RKb[k];
     a.flags = (last ? SF_WAVESP | SF_LAST | SF_TIME : 0) | (first ? SF_FIRST : 0) | (jam ? SF_JAMESON : 0);
-    a.dUg = s->dUg;
     if (first && s->monitor) {
       a.flags |= SF_DIVF;
       a.divF = s->divF[0];
@@ -659,30 +601,7 @@ frg_status enqueue_step(frg_solver *s, int mode, cudaEvent_t *ev = nullptr) {
     // stages after the first follow a stage kernel directly: programmatic
     // dependent launch (not when each launch is timed on its own)
     if (k > 0 && s->pdl && !ev) a.flags |= SF_PDL;
-    if (s->useViscTma) {
-      ViscMaps vm;
-      vm.Uin = first ? s->vm.U : s->vm.Win[(k - 1) & 1];
-      vm.U = s->vm.U;
-      vm.Acc = s->vm.Acc;
-      vm.Wout = s->vm.Wout[k & 1];
-      vm.trOut = s->vm.tr[s->curTr ^ 1];
-      vm.trIn = s->vm.tr[s->curTr];
-      vm.JG = s->vm.JG;
-      vm.det = s->vm.det;
-      vm.nrm = s->vm.nrm;
-      vm.dA = s->vm.dA;
-      vm.nbr = s->vm.nbr;
-      vm.fvn = s->vm.fvn;
-      vm.fvn2 = s->vm.fvn2;
-      const int nTiles = (s->nE + s->ks.vTE - 1) / s->ks.vTE;
-      // the gradient pass one tile per block (measured faster than its
-      // persistent form, which gains nothing from the L2 prefetch), the
-      // stage pass persistent
-      s->ks.vgrad(&a, &vm, nTiles, s->ks.vgradSmem, s->stream);
-      if ((st = post_launch(s))) return st;
-      s->ks.vstage(&a, &vm, std::min(nTiles, s->nSM * s->ks.vstageOcc), s->ks.vstageSmem, s->stream);
-      st = post_launch(s);
-    } else if (s->useTma) {
+    if (s->useTma) {
       TmaMaps mm;
       mm.U = s->mU;
       mm.Acc = s->mAcc;
@@ -780,7 +699,8 @@ frg_status frg_create(const frg_params *params, const frg_mesh *mesh, frg_solver
   KernelKey key{p.nDims, p.order, s->nV, p.precision, s->g.nBndFaces > 0 ? 1 : 0, p.riemannType, p.viscous ? 1 : 0};
   if (!select_kernels(key, s->ks, err)) return fail(FRG_ERR_ARG, "%s", err.c_str());
   s->sstore = p.precision == FRG_FP64 ? 8 : 4;
-  s->nBlk = (s->nE + s->ks.TE - 1) / s->ks.TE;
+  CK(cudaDeviceGetAttribute(&s->nSM, cudaDevAttrMultiProcessorCount, dev));
+  pick_line(s.get());
   CK(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking));
   const size_t nSE = (size_t)s->nV * s->nS * s->L, nFE = (size_t)s->nV * s->nF * s->L;
   if ((st = dalloc(&s->U, nSE)) || (st = dalloc(&s->U0, nSE)) || (st = dalloc(&s->Acc, nSE))) return st;
@@ -843,22 +763,18 @@ frg_status frg_create(const frg_params *params, const frg_mesh *mesh, frg_solver
     return st;
   CK(cudaMallocHost(&s->hostFlag, sizeof(unsigned)));
   if (p.dtType == 0) CK(cudaMemcpy(s->dtDev, &p.dt, sizeof(double), cudaMemcpyHostToDevice));
-  if (s->ks.nTma > 0 && !s->ks.grad) {
+  {
+    const char *pe = getenv("FRG_PDL");
+    s->pdl = !(pe && std::strcmp(pe, "0") == 0);
+  }
+  if (s->ks.nTma > 0) {
     const char *env = getenv("FRG_KERNEL");
     s->useTma = !(env && std::strcmp(env, "generic") == 0);
     if (s->useTma && (st = setup_tma(s.get()))) return st;
-    const char *pe = getenv("FRG_PDL");
-    s->pdl = !(pe && std::strcmp(pe, "0") == 0);
   }
   {
     const char *ge = getenv("FRG_GRAPH");
     s->useGraph = !(ge && std::strcmp(ge, "0") == 0);
-  }
-  CK(cudaDeviceGetAttribute(&s->nSM, cudaDevAttrMultiProcessorCount, dev));
-  if (s->ks.vgrad) {
-    const char *env = getenv("FRG_KERNEL");
-    s->useViscTma = !(env && std::strcmp(env, "generic") == 0);
-    if (s->useViscTma && (st = setup_visc_tma(s.get()))) return st;
   }
   CK(cudaEventCreateWithFlags(&s->noallocOrder, cudaEventDisableTiming));
   {
@@ -1257,7 +1173,7 @@ frg_status frg_calc_residual_noalloc(frg_solver *s, const double *U_dev, double 
   // traces, and for viscous runs the projected viscous fluxes after them
   const size_t one = (size_t)s->nV * s->nF * s->L * s->sstore;
   const size_t oneAligned = (one + 255) & ~size_t(255);
-  const size_t need = one + (s->ks.grad ? oneAligned * (s->visc2 ? 2 : 1) : 0);
+  const size_t need = one + (s->line->grad ? oneAligned * (s->visc2 ? 2 : 1) : 0);
   if (need > kNoAllocScratchBytes)
     return fail(FRG_ERR_ARG, "frg_calc_residual_noalloc: traces need %zu bytes, the scratch array holds %zu", need,
                 kNoAllocScratchBytes);
@@ -1280,17 +1196,17 @@ frg_status frg_calc_residual_noalloc(frg_solver *s, const double *U_dev, double 
   a.trIn = scratch;
   a.divF = divF_dev;
   a.flags = SF_RESIDUAL;
-  if (s->ks.grad) {
+  if (s->line->grad) {
     unsigned char *base = static_cast<unsigned char *>(scratch);
     a.fvnOut = base + oneAligned;
     a.fvnIn = a.fvnOut;
     a.fvn2Out = s->visc2 ? base + 2 * oneAligned : nullptr;
     a.fvn2In = a.fvn2Out;
-    s->ks.grad(&a, s->nBlk, s->ks.smem, st);
+    s->line->grad(&a, s->nBlk, s->line->smem, st);
     CK(cudaGetLastError());
     s->launches += 1;
   }
-  s->ks.stage(&a, s->nBlk, s->ks.smem, st);
+  s->line->stage(&a, s->nBlk, s->line->smem, st);
   CK(cudaGetLastError());
   s->launches += 2;
   return FRG_OK;
@@ -1307,7 +1223,6 @@ frg_status frg_calc_residual(frg_solver *s, int step) {
   a.Uin_d = s->U;
   a.trIn = s->tr[s->curTr];
   a.divF = s->divF[step];
-  a.dUg = s->dUg;
   a.flags = SF_RESIDUAL | SF_WAVESP;
   s->dtFresh = false;  // the wave speeds changed
   if ((st = launch_stage_args(s, a))) return st;
@@ -1394,7 +1309,7 @@ static frg_status step_graph(frg_solver *s, int mode, cudaGraphExec_t *exec, cud
 // Host bookkeeping after a captured step was launched.
 static void step_done(frg_solver *s, int mode) {
   // count the kernels the graph holds
-  s->launches += s->nRK * (s->ks.grad ? 2 : 1) + (s->p.dtType != 0 ? mode : 0) + (s->grp ? 1 : 0);
+  s->launches += s->nRK * (s->line->grad ? 2 : 1) + (s->p.dtType != 0 ? mode : 0) + (s->grp ? 1 : 0);
   s->curTr ^= (s->nRK & 1);
   s->dtFresh = fused_dt(s);
   s->dtLast = s->dtCur;
@@ -1880,6 +1795,7 @@ AdjArgs adj_args(frg_solver *s, const double *Y, const double *gbar) {
   a.dA = static_cast<const double *>(s->dAs);
   a.JG = static_cast<const double *>(s->JG);
   a.detJ = s->detJd;
+  a.invDet = static_cast<const double *>(s->invDetS);
   a.vcjh = s->p.vcjhScheme;
   a.err = s->err;
   a.thetaBar = s->adj->thetaBar;
@@ -2056,7 +1972,7 @@ frg_status boundary_inputs(frg_solver *s, BndIntArgs &b, int kind) {
     a.trIn = s->tr[s->curTr];
     a.dUg = s->dUg;
     a.flags = SF_RESIDUAL;
-    s->ks.grad(&a, s->nBlk, s->ks.smem, s->stream);
+    s->line->grad(&a, s->nBlk, s->line->smem, s->stream);
     if ((st = post_launch(s))) return st;
   }
   if (!s->w1Dev) {

@@ -5,17 +5,13 @@
 #pragma once
 #include "dispatch.h"
 #include "kernels.cuh"
+#include "kernels_line.cuh"
 #include "kernels_tma.cuh"
-#include "kernels_visc_tma.cuh"
 #include "optab_upload.cuh"
 
 namespace frg {
 namespace {
 
-template <class C, typename R, typename S, bool BC, int RS>
-void launch_stage(const void *args, int nBlk, size_t smem, cudaStream_t st) {
-  fr_stage_kernel<C, R, S, BC, RS><<<nBlk, C::NT, smem, st>>>(*static_cast<const StageArgs *>(args));
-}
 // A TMA stage kernel's launch; with SF_PDL it is a programmatic dependent of
 // the previous kernel in the stream (its blocks may start while that kernel's
 // last blocks run, see pdl_wait).
@@ -98,14 +94,6 @@ cudaError_t add_split_variant(KernelSet &k) {
   if (e == cudaSuccess && v.occ < 1) e = cudaErrorInvalidConfiguration;
   return e;
 }
-template <class C, typename R, typename S, bool BC, int RS>
-void launch_stage_visc(const void *args, int nBlk, size_t smem, cudaStream_t st) {
-  fr_stage_visc_kernel<C, R, S, BC, RS><<<nBlk, C::NT, smem, st>>>(*static_cast<const StageArgs *>(args));
-}
-template <class C, typename R, typename S, bool BC>
-void launch_grad(const void *args, int nBlk, size_t smem, cudaStream_t st) {
-  fr_visc_grad_kernel<C, R, S, BC><<<nBlk, C::NT, smem, st>>>(*static_cast<const StageArgs *>(args));
-}
 template <class C, typename R, typename S>
 void launch_trace(const double *U, void *tr, int nE, int nEle, int ldU, int vcjh, cudaStream_t st) {
   long n = (long)C::NF * nE;
@@ -119,26 +107,115 @@ void launch_wavesp(const void *tr, const double *nrmOwn, double *ws, int NF, int
                                                                              NF, nE, ph);
 }
 
-template <class C, typename R, typename S, bool BC, int RS>
+// A line kernel's launch; with SF_PDL a programmatic dependent of the previous
+// kernel in the stream (see pdl_wait).
+template <class K>
+void launch_line(K kernel, const StageArgs &a, int nBlk, int nt, size_t smem, cudaStream_t st) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(nBlk);
+  cfg.blockDim = dim3(nt);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = (a.flags & SF_PDL) ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, kernel, a);
+}
+template <class C, typename R, typename S, bool BC, int RS, int TE, int NT, int MB, bool VISC>
+void launch_line_stage(const void *args, int nBlk, size_t smem, cudaStream_t st) {
+  const StageArgs &a = *static_cast<const StageArgs *>(args);
+  if constexpr (VISC) launch_line(fr_line_visc_stage_kernel<C, R, S, BC, RS, TE, NT, MB>, a, nBlk, NT, smem, st);
+  else launch_line(fr_line_stage_kernel<C, R, S, BC, RS, TE, NT, MB>, a, nBlk, NT, smem, st);
+}
+template <class C, typename R, typename S, bool BC, int TE, int NT, int MB>
+void launch_line_grad(const void *args, int nBlk, size_t smem, cudaStream_t st) {
+  launch_line(fr_line_grad_kernel<C, R, S, BC, TE, NT, MB>, *static_cast<const StageArgs *>(args), nBlk, NT,
+              smem, st);
+}
+template <class K>
+cudaError_t prepare_kernel(K f, size_t smem) {
+  cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+  return e;
+}
+template <class C, typename R, typename S, bool BC, int RS, bool VISC, int TE, int NT, int MB>
+cudaError_t add_line(KernelSet &k) {
+  using T = LineT<C, R, TE, NT>;
+  static_assert(NT % 32 == 0 && NT <= 1024 && T::SMEM <= 227 * 1024, "block shape");
+  KernelSet::LineVariant &v = k.line[k.nLine++];
+  v.stage = &launch_line_stage<C, R, S, BC, RS, TE, NT, MB, VISC>;
+  v.TE = TE;
+  v.rounds = T::LR;
+  v.smem = T::SMEM;
+  if constexpr (VISC) {
+    v.grad = &launch_line_grad<C, R, S, BC, TE, NT, MB>;
+    const cudaError_t e = prepare_kernel(fr_line_grad_kernel<C, R, S, BC, TE, NT, MB>, T::SMEM);
+    return e == cudaSuccess ? prepare_kernel(fr_line_visc_stage_kernel<C, R, S, BC, RS, TE, NT, MB>, T::SMEM) : e;
+  } else {
+    return prepare_kernel(fr_line_stage_kernel<C, R, S, BC, RS, TE, NT, MB>, T::SMEM);
+  }
+}
+// Block shapes of a configuration (elements and threads per block, resident
+// blocks per SM), in the order pick_line tries them.  The first is for meshes that
+// fill the GPU several times: elements as many as keep a warp's accesses whole
+// 128-byte lines where shared memory allows it, threads as many as leave the FP64
+// (FP32) line phase its ~168 (~80) registers, the lines taken in rounds.  Per step
+// of 24,273 (P = 4: 8,000, P = 2: 21,952) periodic hexes, inviscid, us:
+//   P = 2 FP32  32 x 288 x 2: 239   32 x 864: 257   16 x 448 x 2: 260
+//   P = 2 FP64  16 x 224 x 2: 359   32 x 448: 374   32 x 864: 437
+//   P = 3 FP32  32 x 768: 572   16 x 384 x 2: 587   16 x 768: 723   8 x 384 x 2: 799
+//   P = 3 FP64  16 x 384: 882   16 x 256 x 2: 1160  16 x 768: 1214  8 x 384: 1271
+//   P = 4 FP32  16 x 608: 443   8 x 320 x 2: 490    8 x 608: 531
+//   P = 4 FP64  8 x 320: 716    8 x 608: 775 (viscous: 1491 and 1389)
+// The others have a thread for every line of the tile, which is faster where each
+// SM gets one block or none (1,287 hexes, P = 2, FP64, viscous: 16 x 448: 116,
+// 16 x 224: 176), and the last is the narrowest, for meshes too small to give every
+// other SM a wider tile (216 hexes, P = 3, FP64: 4 x 192: 40, 8 x 384: 45,
+// 16 x 384: 76).
+struct LineShape {
+  int TE, NT, MB;
+};
+template <class C, typename R, bool VISC>
+constexpr LineShape line_shape(int tier) {
+  constexpr bool f32 = sizeof(R) == 4;
+  constexpr int n = 2 * C::N1;  // 2D: lines per element
+  constexpr LineShape none{0, 0, 0};
+  constexpr LineShape two[3] = {{32, 32 * n, (f32 ? 768 : 384) / (32 * n)}, {8, (8 * n + 31) & ~31, 1}, none};
+  constexpr LineShape p1[3] = {f32 ? LineShape{32, 384, 2} : LineShape{16, 192, 2}, {8, 96, 1}, none};
+  constexpr LineShape p2[3] = {f32 ? LineShape{32, 288, 2} : LineShape{16, 224, 2}, {16, 448, 1}, {8, 224, 1}};
+  constexpr LineShape p3[3] = {f32 ? LineShape{32, 768, 1} : LineShape{16, 384, 1},
+                               f32 ? LineShape{16, 768, 1} : LineShape{8, 384, 1}, {4, 192, 1}};
+  constexpr LineShape p4[3] = {f32 ? LineShape{16, 608, 1} : LineShape{8, VISC ? 608 : 320, 1}, {8, 608, 1},
+                               {4, 320, 1}};
+  return C::DIM == 2 ? two[tier] : C::P == 1 ? p1[tier] : C::P == 2 ? p2[tier] : C::P == 3 ? p3[tier] : p4[tier];
+}
+template <class C, typename R, typename S, bool BC, int RS, bool VISC, int TIER = 0>
+cudaError_t add_lines(KernelSet &k) {
+  if constexpr (TIER < KernelSet::kMaxLine) {
+    constexpr LineShape sh = line_shape<C, R, VISC>(TIER);
+    if constexpr (sh.TE > 0) {
+      const cudaError_t e = add_line<C, R, S, BC, RS, VISC, sh.TE, sh.NT, (sh.MB > 1 ? sh.MB : 1)>(k);
+      return e == cudaSuccess ? add_lines<C, R, S, BC, RS, VISC, TIER + 1>(k) : e;
+    }
+  }
+  return cudaSuccess;
+}
+template <class C, typename R, typename S, bool BC, int RS, bool VISC>
 bool make_set(KernelSet &k, std::string &err) {
-  using T = Tile<C, R>;
-  k.stage = &launch_stage<C, R, S, BC, RS>;
   k.trace = &launch_trace<C, R, S>;
   k.wavesp = &launch_wavesp<C::DIM, C::NV, S>;
-  k.TE = T::TE;
-  k.NT = C::NT;
-  k.smem = T::SMEM;
-  auto fn = fr_stage_kernel<C, R, S, BC, RS>;
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::SMEM);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+  k.nLine = 0;
+  cudaError_t e = add_lines<C, R, S, BC, RS, VISC>(k);
   if (e == cudaSuccess) {
     // load the trace kernel now (lazy module loading would otherwise load it
     // at its first launch, e.g. inside frg_calc_residual_noalloc)
     cudaFuncAttributes fa;
     e = cudaFuncGetAttributes(&fa, fr_trace_kernel<C, R, S>);
   }
-  if constexpr (C::DIM == 2) {
+  if constexpr (C::DIM == 2 && !VISC) {
     // variant 0 is the default; the others are candidates for frg_autotune
     k.nTma = 0;
     if (e == cudaSuccess) e = add_tma_variant<C, R, S, BC, RS, 0, 128>(k);
@@ -160,82 +237,9 @@ bool make_set(KernelSet &k, std::string &err) {
   return true;
 }
 
-// 3D viscous TMA passes: tiles of 4 (FP32) or 2 (FP64) elements, the 16-byte
-// minimum row of a TMA box; 128 threads for the gradient pass (three blocks
-// per SM), 256 for the stage pass (two blocks per SM, by shared memory)
-template <typename S>
-constexpr int visc_tma_te() { return sizeof(S) == 4 ? 4 : 2; }
-constexpr int kViscGradNT = 256, kViscStageNT = 256;
-template <class C, typename R, typename S, bool BC>
-void launch_visc3_grad(const void *args, const void *maps, int nBlk, size_t smem, cudaStream_t st) {
-  fr_visc3_grad_tma_kernel<C, R, S, BC, visc_tma_te<S>(), kViscGradNT><<<nBlk, kViscGradNT, smem, st>>>(
-      *static_cast<const StageArgs *>(args), *static_cast<const ViscMaps *>(maps));
-}
-template <class C, typename R, typename S, bool BC, int RS>
-void launch_visc3_stage(const void *args, const void *maps, int nBlk, size_t smem, cudaStream_t st) {
-  fr_visc3_stage_tma_kernel<C, R, S, BC, RS, visc_tma_te<S>(), kViscStageNT><<<nBlk, kViscStageNT, smem, st>>>(
-      *static_cast<const StageArgs *>(args), *static_cast<const ViscMaps *>(maps));
-}
-template <class C0, typename R, typename S, bool BC, int RS>
-cudaError_t add_visc3_tma(KernelSet &k) {
-  using C = CfgV<C0>;  // the TMA tiles' point padding
-  constexpr int TE = visc_tma_te<S>();
-  using TG = VGradT<C, R, S, TE, kViscGradNT>;
-  using TS = VStageT<C, R, S, TE, kViscStageNT>;
-  if (TG::SMEM > 227 * 1024 || TS::SMEM > 227 * 1024) return cudaSuccess;  // not offered
-  auto fg = fr_visc3_grad_tma_kernel<C, R, S, BC, TE, kViscGradNT>;
-  auto fs = fr_visc3_stage_tma_kernel<C, R, S, BC, RS, TE, kViscStageNT>;
-  cudaError_t e = cudaFuncSetAttribute(fg, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TG::SMEM);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(fs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TS::SMEM);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(fg, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(fs, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-  if (e != cudaSuccess) return e;
-  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k.vgradOcc, fg, kViscGradNT, TG::SMEM);
-  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k.vstageOcc, fs, kViscStageNT, TS::SMEM);
-  if (e != cudaSuccess) return e;
-  if (k.vgradOcc < 1 || k.vstageOcc < 1) return cudaErrorInvalidConfiguration;
-  k.vgrad = &launch_visc3_grad<C, R, S, BC>;
-  k.vstage = &launch_visc3_stage<C, R, S, BC, RS>;
-  k.vTE = TE;
-  k.vPadG = C::PADG;
-  k.vgradSmem = TG::SMEM;
-  k.vstageSmem = TS::SMEM;
-  return cudaSuccess;
-}
-
-template <class C, typename R, typename S, bool BC, int RS>
-bool make_set_visc(KernelSet &k, std::string &err) {
-  using T = TileV<C, R>;
-  k.stage = &launch_stage_visc<C, R, S, BC, RS>;
-  k.grad = &launch_grad<C, R, S, BC>;
-  k.trace = &launch_trace<C, R, S>;
-  k.wavesp = &launch_wavesp<C::DIM, C::NV, S>;
-  k.TE = T::TE;
-  k.NT = C::NT;
-  k.smem = T::SMEM;
-  auto f1 = fr_stage_visc_kernel<C, R, S, BC, RS>;
-  auto f2 = fr_visc_grad_kernel<C, R, S, BC>;
-  cudaError_t e = cudaFuncSetAttribute(f1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::SMEM);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(f2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::SMEM);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(f1, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(f2, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-  if (e == cudaSuccess) {
-    cudaFuncAttributes fa;  // load the trace kernel now (see make_set)
-    e = cudaFuncGetAttributes(&fa, fr_trace_kernel<C, R, S>);
-  }
-  if constexpr (C::DIM == 3)
-    if (e == cudaSuccess) e = add_visc3_tma<C, R, S, BC, RS>(k);
-  if (e != cudaSuccess) { err = std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e); return false; }
-  return true;
-}
-
 template <class C, typename R, typename S, bool BC, int RS>
 bool make_one(const KernelKey &key, KernelSet &k, std::string &err) {
-  return key.viscous ? make_set_visc<C, R, S, BC, RS>(k, err) : make_set<C, R, S, BC, RS>(k, err);
+  return key.viscous ? make_set<C, R, S, BC, RS, true>(k, err) : make_set<C, R, S, BC, RS, false>(k, err);
 }
 
 template <int DIM, int P, int NV, typename R, typename S>
