@@ -119,46 +119,65 @@ __global__ void fr_timestep_kernel(double *U, const double *U0, const double *di
   else U[i] = U0[i] - coef * divF[i] / detJ[pe] * dtl;
 }
 
-__global__ void fr_norm_kernel(const double *divF, const double *detJ, const double *wvol, int NV, int NS, int nE,
-                               int L, int normType, double *partial, unsigned *ticket, double *out) {
-  // one thread per element: its per-field norm (spt order as the reference),
-  // then per-block totals over elements in index order
-  extern __shared__ double sh[];  // [blockDim][NV]
+// ele::getNormResidual (src/ele.cpp:1882) summed over the elements.  Latency
+// bound (a few MB): a block takes 32 elements, its 8 warps every 8th solution
+// point, so a thread's loads are few and independent; the last block to finish
+// adds the blocks' sums.  One thread per element, with the block's and the final
+// sums taken by one thread, cost a monitored call 152 us more on 4,096 P = 3 hexes.
+constexpr int kNormMaxV = 5;
+__global__ void __launch_bounds__(256) fr_norm_kernel(const double *__restrict__ divF, const double *__restrict__ detJ,
+                                                      const double *__restrict__ wvol, int NV, int NS, int nE, int L,
+                                                      int normType, double *partial, unsigned *ticket, double *out) {
+  __shared__ double sh[8][kNormMaxV];
   __shared__ bool last;
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  for (int v = 0; v < NV; v++) {
-    double r = 0;
-    if (e < nE)
-      for (int s = 0; s < NS; s++) {
-        double dv = divF[((size_t)v * NS + s) * L + e], dj = detJ[(size_t)s * L + e];
-        if (normType == 1) r += fabs(dv) * wvol[s];
-        else if (normType == 2) r += dv * dv / dj * wvol[s];
-        else r = fmax(fabs(dv) / dj, r);
-      }
-    sh[threadIdx.x * NV + v] = r;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
+  const int lane = threadIdx.x & 31, slice = threadIdx.x >> 5, e = blockIdx.x * 32 + lane;
+  auto join = [&](double a, double b) { return normType == 3 ? fmax(a, b) : a + b; };
+  // a warp's total in every lane, then the block's in warp 0
+  auto block_total = [&](const double *r) {
     for (int v = 0; v < NV; v++) {
-      double t = 0;
-      for (int i = 0; i < (int)blockDim.x; i++)
-        t = normType == 3 ? fmax(t, sh[i * NV + v]) : t + sh[i * NV + v];
-      partial[(size_t)blockIdx.x * NV + v] = t;
+      double t = r[v];
+      for (int o = 16; o > 0; o >>= 1) t = join(t, __shfl_xor_sync(0xffffffffu, t, o));
+      if (lane == 0) sh[slice][v] = t;
     }
+    __syncthreads();
+  };
+  double r[kNormMaxV] = {0, 0, 0, 0, 0};
+  if (e < nE)
+    for (int s = slice; s < NS; s += 8) {
+      const double dj = detJ[(size_t)s * L + e], w = wvol[s];
+#pragma unroll
+      for (int v = 0; v < kNormMaxV; v++) {
+        if (v >= NV) break;
+        const double dv = divF[((size_t)v * NS + s) * L + e];
+        if (normType == 1) r[v] += fabs(dv) * w;
+        else if (normType == 2) r[v] += dv * dv / dj * w;
+        else r[v] = fmax(fabs(dv) / dj, r[v]);
+      }
+    }
+  block_total(r);
+  if (threadIdx.x < NV) {
+    double t = sh[0][threadIdx.x];
+    for (int w = 1; w < 8; w++) t = join(t, sh[w][threadIdx.x]);
+    partial[(size_t)blockIdx.x * NV + threadIdx.x] = t;
     __threadfence();
-    last = atomicAdd(ticket, 1u) == gridDim.x - 1;
   }
   __syncthreads();
-  if (!last || threadIdx.x != 0) return;
-  for (int v = 0; v < NV; v++) {
-    double t = 0;
-    for (int b = 0; b < (int)gridDim.x; b++) {
-      double x = ((volatile double *)partial)[(size_t)b * NV + v];
-      t = normType == 3 ? fmax(t, x) : t + x;
-    }
-    out[v] = t;
+  if (threadIdx.x == 0) last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last) return;
+#pragma unroll
+  for (int v = 0; v < kNormMaxV; v++) {
+    r[v] = 0;
+    if (v < NV)
+      for (int b = threadIdx.x; b < (int)gridDim.x; b += 256) r[v] = join(r[v], __ldcg(partial + (size_t)b * NV + v));
   }
-  *ticket = 0;
+  block_total(r);
+  if (threadIdx.x < NV) {
+    double t = sh[0][threadIdx.x];
+    for (int w = 1; w < 8; w++) t = join(t, sh[w][threadIdx.x]);
+    out[threadIdx.x] = t;
+  }
+  if (threadIdx.x == 0) *ticket = 0;
 }
 
 __global__ void fr_to_device_layout(const double *ref, double *dev, int NV, int NPT, int nE, int L) {
@@ -1403,10 +1422,9 @@ frg_status frg_update_host(frg_solver *s, double *U_host, int nsteps) {
 frg_status frg_residual_norm(frg_solver *s, int normType, double *out) {
   if (!s || !out || normType < 1 || normType > 3) return fail(FRG_ERR_ARG, "bad arguments");
   if (!s->divF0Valid) return fail(FRG_ERR_ARG, "no stage-0 residual stored (call frg_calc_residual(0))");
-  const int nb = (s->nE + 255) / 256;
-  fr_norm_kernel<<<nb, 256, 256 * s->nV * sizeof(double), s->stream>>>(s->divF[0], s->detJd, s->wvol, s->nV, s->nS,
-                                                                        s->nE, s->L, normType, s->normPartial, s->ticket,
-                                                                        s->normOut);
+  const int nb = (s->nE + 31) / 32;
+  fr_norm_kernel<<<nb, 256, 0, s->stream>>>(s->divF[0], s->detJd, s->wvol, s->nV, s->nS, s->nE, s->L, normType,
+                                            s->normPartial, s->ticket, s->normOut);
   frg_status st = post_launch(s);
   if (st) return st;
   CK(cudaMemcpyAsync(out, s->normOut, (size_t)s->nV * 8, cudaMemcpyDeviceToHost, s->stream));
