@@ -20,11 +20,21 @@ void launch_adj_face(const AdjArgs &a, cudaStream_t st) {
   const int nb = (int)std::min<long>((n + 255) / 256, kAdjGrid);
   fr_adj_face_kernel<C><<<nb, 256, 0, st>>>(a);
 }
+// A reversed stage; with a.pdl a programmatic dependent of the launch before.
 template <class C, bool BC, int RS>
-void launch_adj_elem(const AdjArgs &a, cudaStream_t st) {
+void launch_adj_stage(const AdjArgs &a, cudaStream_t st) {
   using T = AdjTile<C>;
-  const int nb = (a.nEle + T::TE - 1) / T::TE;
-  fr_adj_elem_kernel<C, BC, RS><<<nb, T::NT, T::SMEM, st>>>(a);
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((a.nEle + T::TE - 1) / T::TE);
+  cfg.blockDim = dim3(T::NT);
+  cfg.dynamicSmemBytes = T::SMEM;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = a.pdl ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, fr_adj_stage_kernel<C, BC, RS>, a);
 }
 template <class C>
 void launch_entropy(const double *U, const double *detJ, const double *wvol, int nE, int L, const Phys &ph,
@@ -91,7 +101,6 @@ bool make_adjv(AdjSet &k, std::string &err) {
   using TV = AdjGradShape<C>;
   k.face = &launch_adj_face<C>;
   k.elem = &launch_adjv_elem<C, BC, RS>;
-  k.TE = T::TE;
   k.elemLaunches = 3;
   if constexpr (C::NV > 1) {
     k.entropy = &launch_entropy<C>;
@@ -111,14 +120,14 @@ template <class C, bool BC, int RS>
 bool make_adj(AdjSet &k, std::string &err) {
   using T = AdjTile<C>;
   k.face = &launch_adj_face<C>;
-  k.elem = &launch_adj_elem<C, BC, RS>;
-  k.TE = T::TE;
+  k.elem = &launch_adj_stage<C, BC, RS>;
+  k.fused = true;
   if constexpr (C::NV > 1) {
     k.entropy = &launch_entropy<C>;
     k.wallp = &launch_wallp<C>;
     k.entropyBlocks = kAdjGrid;
   }
-  cudaError_t e = cudaFuncSetAttribute(fr_adj_elem_kernel<C, BC, RS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  cudaError_t e = cudaFuncSetAttribute(fr_adj_stage_kernel<C, BC, RS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)T::SMEM);
   if (e != cudaSuccess) { err = std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e); return false; }
   return true;

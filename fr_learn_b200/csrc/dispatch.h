@@ -63,8 +63,8 @@ struct AdjSet {
   void (*wallp)(const double *U, const int *nbr, const double *dA, const double *wsurf, int vcjh, int nE, int L,
                 int bcWall, const Phys &ph, double *grad, double *part, cudaStream_t st) = nullptr;
   int entropyBlocks = 0;  // partial sums written by `entropy` (grid size)
-  int TE = 0;             // elements per block of `elem`
   int elemLaunches = 1;   // kernels `elem` launches (three for viscous residuals)
+  bool fused = false;     // `elem` leaves the next stage's face data itself (inviscid)
 };
 bool select_adj_2d(const KernelKey &key, AdjSet &k, std::string &err);
 bool select_adj_3d(const KernelKey &key, AdjSet &k, std::string &err);

@@ -1703,7 +1703,9 @@ struct AdjState {
   AdjSet ks;
   double *seed[2] = {nullptr, nullptr};  // stage seeds dJ/d(divF), ping-pong
   double *lam[2] = {nullptr, nullptr};   // adjoint of a step's final / initial state
-  double *trY = nullptr, *fnbar = nullptr, *ybar = nullptr, *grad = nullptr, *part = nullptr;
+  // traces of the stage state and every side's flux-adjoint share; a fused sweep
+  // reads one set and leaves the next stage's in the other
+  double *trY[2] = {nullptr, nullptr}, *fnbar[2] = {nullptr, nullptr}, *ybar = nullptr, *grad = nullptr, *part = nullptr;
   double *thetaBar = nullptr;
   double *thetaDir = nullptr;  // 5 doubles, device
   // viscous runs: forward gradient, projected fluxes and the pass buffers of
@@ -1738,7 +1740,7 @@ void adj_free(frg_solver *s) {
   AdjState *a = s->adj;
   if (!a) return;
   for (auto &g : a->graphs) cudaGraphExecDestroy(g.second.exec);
-  double *p[] = {a->seed[0], a->seed[1], a->lam[0], a->lam[1], a->trY, a->fnbar, a->ybar, a->grad, a->part,
+  double *p[] = {a->seed[0], a->seed[1], a->lam[0], a->lam[1], a->trY[0], a->trY[1], a->fnbar[0], a->fnbar[1], a->ybar, a->grad, a->part,
                  a->thetaBar, a->thetaDir, a->ckpt, a->stages, a->stages2, a->vg, a->vfvn, a->vfvn2, a->vub,
                  a->vufb, a->vdcb};
   for (double *q : p) if (q) cudaFree(q);
@@ -1783,7 +1785,8 @@ frg_status adj_init(frg_solver *s) {
   const size_t nPart = std::max(a->ks.entropyBlocks, (s->nE + 127) / 128);
   frg_status st;
   if ((st = dalloc(&a->seed[0], nSE)) || (st = dalloc(&a->seed[1], nSE)) || (st = dalloc(&a->lam[0], nSE)) ||
-      (st = dalloc(&a->lam[1], nSE)) || (st = dalloc(&a->trY, nFE)) || (st = dalloc(&a->fnbar, nFE)) ||
+      (st = dalloc(&a->lam[1], nSE)) || (st = dalloc(&a->trY[0], nFE)) || (st = dalloc(&a->fnbar[0], nFE)) ||
+      (a->ks.fused && ((st = dalloc(&a->trY[1], nFE)) || (st = dalloc(&a->fnbar[1], nFE)))) ||
       (st = dalloc(&a->ybar, nSE)) || (st = dalloc(&a->grad, nSE)) || (st = dalloc(&a->part, nPart)) ||
       (st = dalloc(&a->thetaBar, 1)) || (st = dalloc(&a->thetaDir, 5)) ||
       (p.viscous && ((st = dalloc(&a->vg, (size_t)p.nDims * nSE)) || (st = dalloc(&a->vfvn, nFE)) ||
@@ -1806,8 +1809,8 @@ AdjArgs adj_args(frg_solver *s, const double *Y, const double *gbar) {
   a.nEle = s->nE;
   a.Y = Y;
   a.gbar = gbar;
-  a.trY = s->adj->trY;
-  a.fnbar = s->adj->fnbar;
+  a.trY = s->adj->trY[0];
+  a.fnbar = s->adj->fnbar[0];
   a.nbr = s->nbr;
   a.nrm = static_cast<const double *>(s->nrm);
   a.dA = static_cast<const double *>(s->dAs);
@@ -1820,16 +1823,23 @@ AdjArgs adj_args(frg_solver *s, const double *Y, const double *gbar) {
   a.thetaDir = s->adj->thetaDir;
   a.grp = s->grp;
   a.dtGrp = s->grpDt;  // slot 0: the fixed per-group dt
+  StageArgs ops{};
+  set_stage_ops(ops, s->ops);
+  a.op = ops.opd;
   a.v = AdjViscBufs{s->adj->vg, s->adj->vfvn, s->adj->vfvn2, s->adj->vub, s->adj->vufb, s->adj->vdcb,
                     s->visc2 ? 1 : 0};
   a.ph = make_phys(s->p);
   return a;
 }
 
-frg_status adj_launch(frg_solver *s, const AdjArgs &a) {
-  s->adj->ks.face(a, s->stream);
-  frg_status st = post_launch(s);
-  if (st) return st;
+// One residual product; `face`: its traces and flux-adjoint shares first (else
+// the launch before left them).
+frg_status adj_launch(frg_solver *s, const AdjArgs &a, bool face = true) {
+  frg_status st;
+  if (face) {
+    s->adj->ks.face(a, s->stream);
+    if ((st = post_launch(s))) return st;
+  }
   s->adj->ks.elem(a, s->stream);
   s->launches += s->adj->ks.elemLaunches - 1;
   return post_launch(s);
@@ -2316,10 +2326,12 @@ frg_status frg_adjoint_backward(frg_solver *s, const double *lamN_host, const do
     // by launch)
     const int cl0 = cl, cs0 = cs;
     auto reverse = [&]() {
-      int l = cl0, q2 = cs0;
+      int l = cl0, q2 = cs0, x = 0;
+      bool face = true;
       for (int j = m - 1; j >= 0; j--) {
         for (int q = nRK - 1; q >= 0; q--) {
-          AdjArgs a = adj_args(s, seg + nSE * ((size_t)j * nRK + q), ad->seed[q2]);
+          const double *Y = seg + nSE * ((size_t)j * nRK + q);
+          AdjArgs a = adj_args(s, Y, ad->seed[q2]);
           a.mode = ADJ_RK | (q == nRK - 1 ? ADJ_RK_FIRST : 0) | (q == 0 ? ADJ_RK_LAST : 0);
           a.lam = ad->lam[l];
           a.lamNew = ad->lam[l ^ 1];
@@ -2327,8 +2339,20 @@ frg_status frg_adjoint_backward(frg_solver *s, const double *lamN_host, const do
           a.cLam = q == 0 ? s->RKb[nRK - 1] : s->RKb[q - 1];
           a.cY = q == 0 ? 0.0 : s->RKa[q];
           a.dt = dt;
-          frg_status e = adj_launch(s, a);
+          if (ad->ks.fused) {
+            a.trY = ad->trY[x];
+            a.fnbar = ad->fnbar[x];
+            if (j > 0 || q > 0) {  // the stage before lies just below in the slots
+              a.Ynext = Y - nSE;
+              a.trNext = ad->trY[x ^ 1];
+              a.fnNext = ad->fnbar[x ^ 1];
+            }
+            a.pdl = s->pdl && !face;
+            x ^= 1;
+          }
+          frg_status e = adj_launch(s, a, face);
           if (e) return e;
+          face = !ad->ks.fused;
           q2 ^= 1;
         }
         l ^= 1;
