@@ -95,6 +95,16 @@ __device__ __forceinline__ void tmem_free(uint32_t tmem, int ncol) {
   asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(ncol) : "memory");
 }
 
+// 16 accumulator columns of this warp's 32 TMEM lanes (completes with wait::ld)
+__device__ __forceinline__ void tmem_ld16(uint32_t *r, uint32_t addr) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, "
+      "%13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(addr));
+}
+
 __device__ __forceinline__ void tma_load3d(void *dst, const CUtensorMap *m, int x, int y, int z, uint64_t *b) {
   asm volatile(
       "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], "
@@ -162,6 +172,9 @@ __device__ __forceinline__ bool og_wait(uint64_t *b, uint32_t par, volatile int 
   return false;
 }
 
+// ACC: beta is not zero (a variant of its own: the loaded Y takes the registers
+// that the plain drain's 64 columns in flight need).
+template <bool ACC>
 __global__ void __launch_bounds__(kOgThreads, 1)
     fr_op_gemm_tc_kernel(const __grid_constant__ CUtensorMap mX, const float *__restrict__ Bimg, float *Y, int KP,
                          int NP, int M, int ncol, int nA, int ld, int nEle, int nV, float beta, unsigned *err) {
@@ -314,42 +327,67 @@ __global__ void __launch_bounds__(kOgThreads, 1)
       const int t = blockIdx.x + j * gridDim.x;
       if (t >= nTiles) break;
       const int acc = j & 1;
-      if (!og_wait(&sh->accFull[acc], (uint32_t)((j >> 1) & 1), abortF, 0xffffffffu)) break;
-      tc_fence_after();
       const int e = (t % nT) * 128 + 32 * quad + lane, v = t / nT;
       const uint32_t trow = tmem + (uint32_t)(acc * ncol) + ((uint32_t)(32 * quad) << 16);
-      // up to 64 columns in flight per wait (four 16-column loads)
-      for (int c1 = cb; c1 < ce; c1 += 64) {
-        uint32_t r[64];
+      if constexpr (ACC) {
+        // accumulating: 32 columns of Y are loaded at once, the first ones while
+        // the tile is still being multiplied.  (Read, added and stored column by
+        // column, each load behind the previous store, a corrected gradient of
+        // 32,768 P = 3 hexes x 5 fields took 150 us; now 35 us.)  The loads are
+        // unconditional, from clamped addresses, or the compiler joins each with
+        // its store again.
+        const float *const ye = Y + (size_t)v * M * ld + min(e, nEle - 1);
+        float yv[32];
+        auto loadY = [&](int c1) {
+          const float *p = ye + (size_t)min(c1, M - 1) * ld;
 #pragma unroll
-        for (int u = 0; u < 4; u++)
-          if (c1 + 16 * u < ce)
-            asm volatile(
-                "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, "
-                "%13, %14, %15}, [%16];"
-                : "=r"(r[16 * u + 0]), "=r"(r[16 * u + 1]), "=r"(r[16 * u + 2]), "=r"(r[16 * u + 3]),
-                  "=r"(r[16 * u + 4]), "=r"(r[16 * u + 5]), "=r"(r[16 * u + 6]), "=r"(r[16 * u + 7]),
-                  "=r"(r[16 * u + 8]), "=r"(r[16 * u + 9]), "=r"(r[16 * u + 10]), "=r"(r[16 * u + 11]),
-                  "=r"(r[16 * u + 12]), "=r"(r[16 * u + 13]), "=r"(r[16 * u + 14]), "=r"(r[16 * u + 15])
-                : "r"(trow + (uint32_t)(c1 + 16 * u)));
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if (e < nEle) {
-          float *y = Y + ((size_t)v * M + c1) * ld + e;
-          const int nq = min(min(64, ce - c1), M - c1);
-          if (beta == 0.f) {  // plain stores: no read of Y
+          for (int q = 0; q < 32; q++) {
+            asm volatile("ld.global.cs.f32 %0, [%1];" : "=f"(yv[q]) : "l"(p));
+            p += c1 + q < M - 1 ? ld : 0;
+          }
+        };
+        loadY(cb);
+        if (!og_wait(&sh->accFull[acc], (uint32_t)((j >> 1) & 1), abortF, 0xffffffffu)) break;
+        tc_fence_after();
+        for (int c1 = cb; c1 < ce; c1 += 32) {
+          if (c1 > cb) loadY(c1);
+          uint32_t r[32];
+#pragma unroll
+          for (int u = 0; u < 2; u++)
+            if (c1 + 16 * u < ce) tmem_ld16(r + 16 * u, trow + (uint32_t)(c1 + 16 * u));
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          if (e < nEle) {
+            float *y = Y + ((size_t)v * M + c1) * ld + e;
+            const int nq = min(min(32, ce - c1), M - c1);
+#pragma unroll
+            for (int q = 0; q < 32; q++)
+              if (q < nq) __stcs(y + (size_t)q * ld, fmaf(beta, yv[q], __uint_as_float(r[q])));
+          }
+        }
+        tc_fence_before();
+        mbar_arrive(&sh->accEmpty[acc]);
+      } else {
+        if (!og_wait(&sh->accFull[acc], (uint32_t)((j >> 1) & 1), abortF, 0xffffffffu)) break;
+        tc_fence_after();
+        // up to 64 columns in flight per wait (four 16-column loads)
+        for (int c1 = cb; c1 < ce; c1 += 64) {
+          uint32_t r[64];
+#pragma unroll
+          for (int u = 0; u < 4; u++)
+            if (c1 + 16 * u < ce) tmem_ld16(r + 16 * u, trow + (uint32_t)(c1 + 16 * u));
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          if (e < nEle) {
+            float *y = Y + ((size_t)v * M + c1) * ld + e;
+            const int nq = min(min(64, ce - c1), M - c1);
 #pragma unroll
             for (int q = 0; q < 64; q++)
               if (q < nq) __stcs(y + (size_t)q * ld, __uint_as_float(r[q]));
-          } else {
-#pragma unroll
-            for (int q = 0; q < 64; q++)
-              if (q < nq) y[(size_t)q * ld] = fmaf(beta, y[(size_t)q * ld], __uint_as_float(r[q]));
           }
         }
+        // the accumulator is free for the MMAs of tile j + 2
+        tc_fence_before();
+        mbar_arrive(&sh->accEmpty[acc]);
       }
-      // the accumulator is free for the MMAs of tile j + 2
-      tc_fence_before();
-      mbar_arrive(&sh->accEmpty[acc]);
     }
   }
   tc_fence_before();
@@ -433,10 +471,11 @@ cudaError_t launch_op_gemm(const CUtensorMap &mX, const float *Bimg, float *Y, i
     std::lock_guard<std::mutex> lk(mu);
     auto it = smCount.find(dev);
     if (it == smCount.end()) {
-      e = cudaFuncSetAttribute(fr_op_gemm_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-      if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(fr_op_gemm_tc_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                 cudaSharedmemCarveoutMaxShared);
+      for (auto f : {&fr_op_gemm_tc_kernel<false>, &fr_op_gemm_tc_kernel<true>}) {
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+        if (e == cudaSuccess)
+          e = cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+      }
       if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nSM, cudaDevAttrMultiProcessorCount, dev);
       if (e != cudaSuccess) return e;
       smCount[dev] = nSM;
@@ -445,11 +484,12 @@ cudaError_t launch_op_gemm(const CUtensorMap &mX, const float *Bimg, float *Y, i
     }
   }
   int occ = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fr_op_gemm_tc_kernel, kOgThreads, smem);
+  auto kernel = beta == 0.f ? &fr_op_gemm_tc_kernel<false> : &fr_op_gemm_tc_kernel<true>;
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, kOgThreads, smem);
   if (e != cudaSuccess) return e;
   const int nTiles = (nEle + 127) / 128 * nV;
   const int grid = std::max(1, std::min(nTiles, nSM * std::max(occ, 1)));
-  fr_op_gemm_tc_kernel<<<grid, kOgThreads, smem, st>>>(mX, Bimg, Y, KP, NP, M, ncol, nA, ld, nEle, nV, beta, err);
+  kernel<<<grid, kOgThreads, smem, st>>>(mX, Bimg, Y, KP, NP, M, ncol, nA, ld, nEle, nV, beta, err);
   return cudaGetLastError();
 }
 
