@@ -457,7 +457,7 @@ __device__ __forceinline__ void line_stage_end(const StageArgs &a, const OpTab<R
         for (int v = 0; v < NV; v++) u0[r][v] = __ldcg(a.U0 + g0 + v * gs);
       }
       idet[r] = (R)__ldg(static_cast<const S *>(a.invDet) + (size_t)s * (unsigned)a.nE + e0 + e);
-      dtl[r] = a.grp ? a.dt[a.grp[e0 + e]] : a.dtLocal ? a.dt[e0 + e] : __ldg(a.dt);
+      dtl[r] = a.grp ? a.dt[a.grp[e0 + e]] : a.dtLocal ? a.dt[e0 + e] : stage_dt(a);
     }
   }
   __syncthreads();
@@ -484,7 +484,7 @@ __device__ __forceinline__ void line_stage_end(const StageArgs &a, const OpTab<R
     }
   }
   if (resid) return;
-  if ((a.flags & SF_TIME) && !a.grp && blockIdx.x == 0 && threadIdx.x == 0) *a.time += __ldg(a.dt);
+  if ((a.flags & SF_TIME) && !a.grp && blockIdx.x == 0 && threadIdx.x == 0) *a.time += stage_dt(a);
   __syncthreads();
 #pragma unroll 1
   for (int r = 0; r < T::LR; r++) {

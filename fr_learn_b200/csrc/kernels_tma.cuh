@@ -28,7 +28,8 @@ enum : unsigned { ERRF_TIMEOUT = 8u, ERRF_ALIGN = 16u };
 
 // Tensor maps of one stage launch (all 2D: [rows][element stride]).
 struct TmaMaps {
-  CUtensorMap U;      // double [NV*NS]: stage-0 input, U0, final state
+  CUtensorMap U;      // double [NV*NS]: stage-0 input, U0
+  CUtensorMap Uout;   // double [NV*NS]: final state (U, unless the caller keeps every stage state)
   CUtensorMap Acc;    // double [NV*NS]: RK accumulator
   CUtensorMap Win;    // S [NV*NS]: stage input (stages >= 1)
   CUtensorMap Wout;   // S [NV*NS]: next stage state
@@ -100,6 +101,15 @@ __device__ __forceinline__ void pdl_launch_dependents() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// The global dt.  The previous step's last stage wrote it, possibly in the grid
+// that this one is a programmatic dependent of, so the load must stay behind
+// pdl_wait (a read-only load may be moved ahead of it).
+__device__ __forceinline__ double stage_dt(const StageArgs &a) {
+  double x;
+  asm volatile("ld.global.cg.f64 %0, [%1];" : "=d"(x) : "l"(a.dt) : "memory");
+  return x;
+}
 
 // First stage of a step with the fused dt: the slot the last stage will
 // minimise the next dt into starts at a huge value (the bytes 0x7F, as a
@@ -524,7 +534,7 @@ __global__ void __launch_bounds__(NTV, (TileT<C, R, S, TEV, NTV>::MINB))
   if (tid == 0) tma_issue_tile<C, R, S, TE>(m, nd, b, e0, bar, 2);
 
   // the global dt, fetched while the tiles are in flight
-  const double dtG = (a.dtLocal || a.grp) ? 0.0 : __ldg(a.dt);
+  const double dtG = (a.dtLocal || a.grp) ? 0.0 : stage_dt(a);
 
   // ---- group 0: gathers of neighbour traces, then phase A
   bool ok = mbar_wait(&bar[0], 0);
@@ -546,7 +556,7 @@ __global__ void __launch_bounds__(NTV, (TileT<C, R, S, TEV, NTV>::MINB))
   fence_proxy_async();
   __syncthreads();
   if (tid == 0) {
-    if (last) tma_store2d(&m.U, e0, 0, b.U0);
+    if (last) tma_store2d(&m.Uout, e0, 0, b.U0);
     else {
       tma_store2d(&m.Wout, e0, 0, b.Us);
       if (!jam) tma_store2d(&m.Acc, e0, 0, b.Acc);
@@ -676,7 +686,7 @@ __global__ void __launch_bounds__(NT, (PipeT<C, R, S, TEV, NT, NB>::MINB))
   pdl_wait();  // the previous stage has finished: its outputs are visible
   stage_dt_reset(a);
   if (tid == 0) tma_issue_tile<C, R, S, TE>(m, nd, slot(0), blockIdx.x * TE, &bar[0], 2);
-  const double dtG = (a.dtLocal || a.grp) ? 0.0 : __ldg(a.dt);
+  const double dtG = (a.dtLocal || a.grp) ? 0.0 : stage_dt(a);
   double dtMin = INFINITY;
   const bool dtn = flags & SF_DTNEXT;
   int prevE0 = -1;  // the previous tile's first element, for its deferred dt
@@ -732,7 +742,7 @@ __global__ void __launch_bounds__(NT, (PipeT<C, R, S, TEV, NT, NB>::MINB))
     fence_proxy_async();
     __syncthreads();
     if (tid == 0) {
-      if (last) tma_store2d(&m.U, e0, 0, b.U0);
+      if (last) tma_store2d(&m.Uout, e0, 0, b.U0);
       else {
         tma_store2d(&m.Wout, e0, 0, b.Us);
         if (!jam) tma_store2d(&m.Acc, e0, 0, b.Acc);
@@ -905,7 +915,7 @@ __global__ void __launch_bounds__(NT, (SplitT<C, R, S, TEV, NT>::MINB))
     issue_slot(slot(0), blockIdx.x * TE, &bar[0], 2);
     if (needUg) issue_u(slot(0), blockIdx.x * TE);
   }
-  const double dtG = (a.dtLocal || a.grp) ? 0.0 : __ldg(a.dt);
+  const double dtG = (a.dtLocal || a.grp) ? 0.0 : stage_dt(a);
   double dtMin = INFINITY;
   const bool dtn = flags & SF_DTNEXT;
   int prevE0 = -1;  // the previous tile's first element, for its deferred dt
@@ -995,7 +1005,7 @@ __global__ void __launch_bounds__(NT, (SplitT<C, R, S, TEV, NT>::MINB))
     fence_proxy_async();
     __syncthreads();
     if (tid == 0) {
-      if (last) tma_store2d(&m.U, e0, 0, b.U0);
+      if (last) tma_store2d(&m.Uout, e0, 0, b.U0);
       else {
         tma_store2d(&m.Wout, e0, 0, b.Us);
         if (!jam) tma_store2d(&m.Acc, e0, 0, b.Acc);
