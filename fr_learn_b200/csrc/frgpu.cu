@@ -1963,23 +1963,24 @@ frg_status state_to_host(frg_solver *s, const double *dev, double *host) {
   return FRG_OK;
 }
 
-// One RK step from U (on entry U_n, on exit U_{n+1}) keeping every stage
-// state: Y[0] receives a copy of U_n and Y[k] (k = 1..nRK-1) the state stage
-// k's residual is evaluated at.  Same kernels and arithmetic as frg_update:
-// the TMA stage kernel where the update uses it (stage states through tensor
-// maps made for the Y slots), else the generic one.  Traces of U must be
-// current on entry (tr[curTr]) and are current on exit.
-frg_status step_keep_stages(frg_solver *s, double *const *Y, bool advanceTime = false) {
-  const size_t nSE = (size_t)s->nV * s->nS * s->L;
-  CK(cudaMemcpyAsync(Y[0], s->U, nSE * 8, cudaMemcpyDeviceToDevice, s->stream));
+// One RK step keeping every stage state: on entry Y[0] holds U_n; Y[k] (k =
+// 1..nRK-1) receives the state stage k's residual is evaluated at and Uend U_{n+1}
+// (the next step's Y[0], or U).  Same kernels and arithmetic as frg_update: the
+// TMA stage kernel where the update uses it (states through tensor maps made for
+// the slots), else the line kernels.  Traces of U_n must be current on entry
+// (tr[curTr]); those of U_{n+1} are on exit.  `chained`: the kernel before on the
+// stream is the last stage of the step before.
+frg_status step_keep_stages(frg_solver *s, double *const *Y, double *Uend, bool chained, bool advanceTime = false) {
   frg_status st;
   const int nRK = s->nRK;
-  CUtensorMap mY[8];
-  if (s->useTma)
-    for (int k = 1; k < nRK; k++)
-      if ((st = make_map(&mY[k], Y[k], CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 8, s->nV * s->nS, s->L,
-                         s->ks.tma[s->tmaVar].TE)))
+  CUtensorMap mY[8], mEnd;
+  if (s->useTma) {
+    const int rows = s->nV * s->nS, TE = s->ks.tma[s->tmaVar].TE;
+    for (int k = 0; k <= nRK; k++)
+      if ((st = make_map(k < nRK ? &mY[k] : &mEnd, k < nRK ? Y[k] : Uend, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 8, rows,
+                         s->L, TE)))
         return st;
+  }
   for (int k = 0; k < nRK; k++) {
     StageArgs a = base_args(s);
     const bool first = k == 0, last = k == nRK - 1;
@@ -1988,14 +1989,19 @@ frg_status step_keep_stages(frg_solver *s, double *const *Y, bool advanceTime = 
     a.aNext = last ? 0.0 : s->RKa[k + 1];
     a.bCur = s->RKb[k];
     a.flags = (last ? SF_LAST : 0) | (first ? SF_FIRST : 0) | (last && advanceTime ? SF_TIME : 0);
+    const bool groups = first && advanceTime && s->grp;
+    if (groups && (st = launch_group_step(s))) return st;
+    if (s->pdl && (k > 0 || (chained && !groups))) a.flags |= SF_PDL;
     a.Acc = s->Acc;
-    if (first && advanceTime && s->grp && (st = launch_group_step(s))) return st;
+    a.Uin_d = first ? Y[0] : nullptr;
+    a.Uin_s = first ? nullptr : Y[k];
+    a.U0 = Y[0];
+    a.Uout = Uend;
+    a.Wout = last ? nullptr : Y[k + 1];
     if (s->useTma) {
-      a.Uin_d = first ? s->U : nullptr;
-      a.Uin_s = first ? nullptr : Y[k];
       TmaMaps mm;
-      mm.U = s->mU;
-      mm.Uout = s->mU;
+      mm.U = mY[0];
+      mm.Uout = mEnd;
       mm.Acc = s->mAcc;
       mm.Win = first ? s->mW[0] : mY[k];
       mm.Wout = last ? s->mW[0] : mY[k + 1];
@@ -2010,15 +2016,23 @@ frg_status step_keep_stages(frg_solver *s, double *const *Y, bool advanceTime = 
       tv.launch(&a, &mm, s->nBlkTma, tv.smem, s->stream);
       st = post_launch(s);
     } else {
-      a.Uin_d = first ? Y[0] : nullptr;
-      a.Uin_s = first ? nullptr : Y[k];
-      a.U0 = Y[0];
-      a.Uout = s->U;
-      a.Wout = last ? nullptr : Y[k + 1];
       st = launch_stage_args(s, a);
     }
     if (st) return st;
     s->curTr ^= 1;
+  }
+  return FRG_OK;
+}
+// m steps from U to U, every stage state in the slots `seg` ([step][stage]).
+frg_status steps_keep_stages(frg_solver *s, double *seg, int m, bool advanceTime = false) {
+  const size_t nSE = (size_t)s->nV * s->nS * s->L;
+  CK(cudaMemcpyAsync(seg, s->U, nSE * 8, cudaMemcpyDeviceToDevice, s->stream));
+  std::vector<double *> Y(s->nRK);
+  for (int n = 0; n < m; n++) {
+    for (int q = 0; q < s->nRK; q++) Y[q] = seg + nSE * ((size_t)n * s->nRK + q);
+    frg_status st = step_keep_stages(s, Y.data(), n + 1 < m ? seg + nSE * (size_t)(n + 1) * s->nRK : s->U, n > 0,
+                                     advanceTime);
+    if (st) return st;
   }
   return FRG_OK;
 }
@@ -2292,12 +2306,8 @@ frg_status frg_adjoint_forward(frg_solver *s, int nsteps, int checkpointEvery) {
   if (keepAll) {
     CK(cudaMemcpyAsync(a->ckpt, s->U, nSE * 8, cudaMemcpyDeviceToDevice, s->stream));
     if ((st = ensure_traces(s))) return st;
-    std::vector<double *> Y(s->nRK);
-    for (int n = 0; n < nsteps; n++) {
-      for (int q = 0; q < s->nRK; q++) Y[q] = a->stages + nSE * ((size_t)n * s->nRK + q);
-      if ((st = step_keep_stages(s, Y.data(), true))) return st;
-      s->iter++;
-    }
+    if ((st = steps_keep_stages(s, a->stages, nsteps, true))) return st;
+    s->iter += nsteps;
     s->trValid = true;
     s->dtFresh = false;
   } else {
@@ -2362,15 +2372,7 @@ frg_status frg_adjoint_backward(frg_solver *s, const double *lamN_host, const do
     frg_status e = ensure_traces(s);
     if (e) return e;
     const int tr0 = s->curTr;
-    e = adj_replay(s, {2 * b, m, tr0, 0}, [&]() {
-      std::vector<double *> Y(nRK);
-      for (int j = 0; j < m; j++) {
-        for (int q = 0; q < nRK; q++) Y[q] = seg + nSE * ((size_t)j * nRK + q);
-        frg_status e2 = step_keep_stages(s, Y.data());
-        if (e2) return e2;
-      }
-      return FRG_OK;
-    });
+    e = adj_replay(s, {2 * b, m, tr0, 0}, [&]() { return steps_keep_stages(s, seg, m); });
     if (e) return e;
     s->curTr = tr0 ^ ((m * nRK) & 1);
     return FRG_OK;
