@@ -2279,13 +2279,16 @@ frg_status frg_adjoint_forward(frg_solver *s, int nsteps, int checkpointEvery) {
   const int k = keepAll ? nsteps : std::min(checkpointEvery, nsteps);
   const int nCkpt = (nsteps + k - 1) / k;  // checkpoints at 0, k, ..., plus U_N
   CK(cudaStreamSynchronize(s->stream));
-  adj_drop_graphs(a);  // they name the stage slots of the last run's layout
+  // (the segment graphs name the stage slots and are kept with them: every other
+  // thing they hold -- metrics, trace and adjoint buffers -- lives as long as the
+  // handle, and what changes it drops them)
   if (a->ckpt && a->ckptCap < nCkpt + 1) { cudaFree(a->ckpt); a->ckpt = nullptr; }
   if (!a->ckpt) {
     if ((st = dalloc(&a->ckpt, nSE * (nCkpt + 1)))) return st;
     a->ckptCap = nCkpt + 1;
   }
   if (a->stages && a->stagesCap < k) {
+    adj_drop_graphs(a);
     cudaFree(a->stages);
     cudaFree(a->stages2);
     a->stages = a->stages2 = nullptr;
@@ -2313,7 +2316,7 @@ frg_status frg_adjoint_forward(frg_solver *s, int nsteps, int checkpointEvery) {
   } else {
     for (int n = 0; n < nsteps; n += k) {
       CK(cudaMemcpyAsync(a->ckpt + nSE * (n / k), s->U, nSE * 8, cudaMemcpyDeviceToDevice, s->stream));
-      if ((st = frg_update(s, std::min(k, nsteps - n)))) return st;
+      if ((st = enqueue_updates(s, std::min(k, nsteps - n)))) return st;
     }
   }
   CK(cudaMemcpyAsync(a->ckpt + nSE * nCkpt, s->U, nSE * 8, cudaMemcpyDeviceToDevice, s->stream));
