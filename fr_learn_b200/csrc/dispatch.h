@@ -18,6 +18,8 @@ struct KernelSet {
   // traces of a double state: nE is the element stride of the trace array,
   // nEle the number of real elements, ldU the element stride of U
   void (*trace)(const double *U, void *tr, int nE, int nEle, int ldU, int vcjh, cudaStream_t st) = nullptr;
+  // a state from the reference layout, with its traces
+  void (*import)(const double *ref, double *U, void *tr, int nEle, int L, int vcjh, cudaStream_t st) = nullptr;
   void (*wavesp)(const void *tr, const double *nrmOwn, double *ws, int NF, int nE, const Phys &ph,
                  cudaStream_t st) = nullptr;
   // the fused-update stage kernel with TMA tile movement (2D inviscid), in

@@ -180,23 +180,25 @@ __global__ void __launch_bounds__(256) fr_norm_kernel(const double *__restrict__
   if (threadIdx.x == 0) *ticket = 0;
 }
 
-__global__ void fr_to_device_layout(const double *ref, double *dev, int NV, int NPT, int nE, int L) {
-  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;  // ref index
-  const long total = (long)NV * NPT * nE;
-  if (i >= total) return;
-  const int v = (int)(i % NV);
-  const long pe = i / NV;  // pt * nE + e
-  const long pt = pe / nE, e = pe - pt * nE;
-  dev[((long)v * NPT + pt) * L + e] = ref[i];
+// Between the reference's layout [point][ele][field] and the device's
+// [field][point][L]: a thread moves one point's fields of one element (one value
+// per thread, its indices by 64-bit divisions, was bound by those).
+__global__ void __launch_bounds__(128) fr_to_device_layout(const double *__restrict__ ref, double *__restrict__ dev,
+                                                           int NV, int NPT, int nE, int L) {
+  const int e = blockIdx.x * 128 + threadIdx.x, pt = blockIdx.y;
+  if (e >= nE) return;
+  const double *r = ref + ((size_t)pt * nE + e) * NV;
+  for (int v = 0; v < NV; v++) dev[((size_t)v * NPT + pt) * L + e] = r[v];
 }
-__global__ void fr_to_ref_layout(const double *dev, double *ref, int NV, int NPT, int nE, int L) {
-  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;  // ref index
-  const long total = (long)NV * NPT * nE;
-  if (i >= total) return;
-  const int v = (int)(i % NV);
-  const long pe = i / NV;
-  const long pt = pe / nE, e = pe - pt * nE;
-  ref[i] = dev[((long)v * NPT + pt) * L + e];
+// flag: if not null, the flag word is passed on with the state (to pinned host
+// memory: it needs no copy of its own).
+__global__ void __launch_bounds__(128) fr_to_ref_layout(const double *__restrict__ dev, double *__restrict__ ref, int NV,
+                                                        int NPT, int nE, int L, const unsigned *err, unsigned *flag) {
+  const int e = blockIdx.x * 128 + threadIdx.x, pt = blockIdx.y;
+  if (flag && e == 0 && pt == 0) *flag = *err;
+  if (e >= nE) return;
+  double *r = ref + ((size_t)pt * nE + e) * NV;
+  for (int v = 0; v < NV; v++) r[v] = dev[((size_t)v * NPT + pt) * L + e];
 }
 template <typename S>
 __global__ void fr_cast_kernel(const double *in, S *out, long n) {
@@ -1061,6 +1063,12 @@ frg_status frg_apply_operator(frg_solver *s, int which, int dim, const float *X,
   return FRG_OK;
 }
 
+// A device array of npt points per element in the reference's layout (dst: device
+// or pinned host memory); with `flag` the flag word too.
+static void to_ref_layout(frg_solver *s, const double *src, double *dst, int npt, unsigned *flag = nullptr) {
+  fr_to_ref_layout<<<dim3((s->nE + 127) / 128, npt), 128, 0, s->stream>>>(src, dst, s->nV, npt, s->nE, s->L, s->err,
+                                                                          flag);
+}
 static frg_status ref_scratch(frg_solver *s, size_t n) {
   if (!s->scratchRef) {
     size_t big = (size_t)s->nV * std::max(s->nS, s->nF) * s->nE;
@@ -1078,9 +1086,8 @@ frg_status frg_upload(frg_solver *s, int array, const double *host) {
   if (st) return st;
   const size_t n = (size_t)s->nV * s->nS * s->nE;
   CK(cudaMemcpyAsync(s->scratchRef, host, n * 8, cudaMemcpyHostToDevice, s->stream));
-  fr_to_device_layout<<<(unsigned)((n + 255) / 256), 256, 0, s->stream>>>(s->scratchRef,
-                                                                         array == FRG_U0 ? s->U0 : s->U, s->nV,
-                                                                         s->nS, s->nE, s->L);
+  fr_to_device_layout<<<dim3((s->nE + 127) / 128, s->nS), 128, 0, s->stream>>>(
+      s->scratchRef, array == FRG_U0 ? s->U0 : s->U, s->nV, s->nS, s->nE, s->L);
   if ((st = post_launch(s))) return st;
   if (array == FRG_U_SPTS) s->trValid = false;
   CK(cudaStreamSynchronize(s->stream));
@@ -1141,7 +1148,7 @@ frg_status frg_download(frg_solver *s, int array, int stage, double *host) {
       return fail(FRG_ERR_ARG, "unknown array %d", array);
   }
   const size_t n = (size_t)s->nV * npt * s->nE;
-  fr_to_ref_layout<<<(unsigned)((n + 255) / 256), 256, 0, s->stream>>>(src, s->scratchRef, s->nV, npt, s->nE, s->L);
+  to_ref_layout(s, src, s->scratchRef, npt);
   if ((st = post_launch(s))) return st;
   CK(cudaMemcpyAsync(host, s->scratchRef, n * 8, cudaMemcpyDeviceToHost, s->stream));
   CK(cudaStreamSynchronize(s->stream));
@@ -1454,6 +1461,7 @@ frg_status frg_update(frg_solver *s, int nsteps) {
   return check_flags(s);
 }
 
+constexpr size_t kDirectBytes = size_t(256) << 10;
 // Upload, steps, download and the flag word on the handle's stream with one
 // synchronisation at the end (the host waits once per call, not after each
 // part).  The state is written back even when a flag is raised: the
@@ -1470,19 +1478,24 @@ frg_status frg_update_host(frg_solver *s, double *U_host, int nsteps) {
   if ((st = ref_scratch(s, 0))) return st;
   const size_t n = (size_t)s->nV * s->nS * s->nE;
   CK(cudaMemcpyAsync(s->scratchRef, U_host, n * 8, cudaMemcpyHostToDevice, s->stream));
-  fr_to_device_layout<<<(unsigned)((n + 255) / 256), 256, 0, s->stream>>>(s->scratchRef, s->U, s->nV, s->nS, s->nE,
-                                                                         s->L);
+  s->ks.import(s->scratchRef, s->U, s->tr[s->curTr], s->nE, s->L, s->p.vcjhScheme, s->stream);
   if ((st = post_launch(s))) return st;
-  s->trValid = false;
+  s->trValid = true;
   if ((st = enqueue_updates(s, nsteps))) {
     cudaStreamSynchronize(s->stream);  // the upload still reads U_host
     return st;
   }
-  fr_to_ref_layout<<<(unsigned)((n + 255) / 256), 256, 0, s->stream>>>(s->U, s->scratchRef, s->nV, s->nS, s->nE,
-                                                                       s->L);
+  // the flag word goes to the host with the state; a small state goes straight
+  // into the caller's buffer where that is pinned (the copy's own latency, about
+  // 5 us, is more than its bytes take: below kDirectBytes)
+  double *direct = nullptr;
+  cudaPointerAttributes at;
+  if (n * 8 <= kDirectBytes && cudaPointerGetAttributes(&at, U_host) == cudaSuccess && at.type == cudaMemoryTypeHost)
+    direct = static_cast<double *>(at.devicePointer);
+  cudaGetLastError();  // (an unknown pointer is no error)
+  to_ref_layout(s, s->U, direct ? direct : s->scratchRef, s->nS, s->hostFlag);
   if ((st = post_launch(s))) return st;
-  CK(cudaMemcpyAsync(s->hostFlag, s->err, sizeof(unsigned), cudaMemcpyDeviceToHost, s->stream));
-  CK(cudaMemcpyAsync(U_host, s->scratchRef, n * 8, cudaMemcpyDeviceToHost, s->stream));
+  if (!direct) CK(cudaMemcpyAsync(U_host, s->scratchRef, n * 8, cudaMemcpyDeviceToHost, s->stream));
   CK(cudaStreamSynchronize(s->stream));
   return flags_status(s, *s->hostFlag);
 }
@@ -1948,15 +1961,15 @@ frg_status state_to_dev(frg_solver *s, const double *host, double *dev) {
   if (st) return st;
   const size_t n = (size_t)s->nV * s->nS * s->nE;
   CK(cudaMemcpyAsync(s->scratchRef, host, n * 8, cudaMemcpyHostToDevice, s->stream));
-  fr_to_device_layout<<<(unsigned)((n + 255) / 256), 256, 0, s->stream>>>(s->scratchRef, dev, s->nV, s->nS, s->nE,
-                                                                         s->L);
+  fr_to_device_layout<<<dim3((s->nE + 127) / 128, s->nS), 128, 0, s->stream>>>(s->scratchRef, dev, s->nV, s->nS, s->nE,
+                                                                              s->L);
   return post_launch(s);
 }
 frg_status state_to_host(frg_solver *s, const double *dev, double *host) {
   frg_status st = ref_scratch(s, 0);
   if (st) return st;
   const size_t n = (size_t)s->nV * s->nS * s->nE;
-  fr_to_ref_layout<<<(unsigned)((n + 255) / 256), 256, 0, s->stream>>>(dev, s->scratchRef, s->nV, s->nS, s->nE, s->L);
+  to_ref_layout(s, dev, s->scratchRef, s->nS);
   if ((st = post_launch(s))) return st;
   CK(cudaMemcpyAsync(host, s->scratchRef, n * 8, cudaMemcpyDeviceToHost, s->stream));
   CK(cudaStreamSynchronize(s->stream));

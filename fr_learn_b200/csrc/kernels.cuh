@@ -285,6 +285,39 @@ __global__ void fr_trace_kernel(const double *__restrict__ U, S *__restrict__ tr
   }
 }
 
+// A state in the reference's layout [spt][ele][field] into the device's, and the
+// traces of it, in one launch: block row y < NS converts solution point y, the
+// others form flux point y - NS's traces straight from the reference layout.
+template <class C, typename R, typename S>
+__global__ void __launch_bounds__(128) fr_import_kernel(const double *__restrict__ ref, double *__restrict__ U,
+                                                        S *__restrict__ tr, int nEle, int L, int vcjh) {
+  constexpr int NS = C::NS, NF = C::NF, NV = C::NV, N1 = C::N1;
+  const int e = blockIdx.x * 128 + threadIdx.x, y = blockIdx.y;
+  if (e >= nEle) return;
+  if (y < NS) {
+    const double *r = ref + ((size_t)y * nEle + e) * NV;
+#pragma unroll
+    for (int v = 0; v < NV; v++) U[(size_t)(v * NS + y) * L + e] = r[v];
+    return;
+  }
+  const OpTab<R> &op = optab<R>(vcjh, C::P);
+  const int f = y - NS;
+  int dir, side, s0, st;
+  fpt_line<C>(f, dir, side, s0, st);
+  R t[NV];
+#pragma unroll
+  for (int v = 0; v < NV; v++) t[v] = 0;
+#pragma unroll
+  for (int j = 0; j < N1; j++) {
+    const double *r = ref + ((size_t)(s0 + j * st) * nEle + e) * NV;
+    const R l = op.lag[side][j];
+#pragma unroll
+    for (int v = 0; v < NV; v++) t[v] += l * (R)r[v];
+  }
+#pragma unroll
+  for (int v = 0; v < NV; v++) tr[(size_t)(v * NF + f) * L + e] = (S)t[v];
+}
+
 // ele::calcWaveSpFpts (src/ele.cpp:1031-1084) for every flux point.
 template <int DIM, int NV, typename S>
 __global__ void fr_wavesp_kernel(const S *__restrict__ tr, const double *__restrict__ nrmOwn, double *waveSp,

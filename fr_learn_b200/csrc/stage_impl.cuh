@@ -100,6 +100,11 @@ void launch_trace(const double *U, void *tr, int nE, int nEle, int ldU, int vcjh
   fr_trace_kernel<C, R, S><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(U, static_cast<S *>(tr), nE, nEle, ldU,
                                                                          vcjh);
 }
+template <class C, typename R, typename S>
+void launch_import(const double *ref, double *U, void *tr, int nEle, int L, int vcjh, cudaStream_t st) {
+  fr_import_kernel<C, R, S><<<dim3((nEle + 127) / 128, C::NS + C::NF), 128, 0, st>>>(ref, U, static_cast<S *>(tr), nEle,
+                                                                                   L, vcjh);
+}
 template <int DIM, int NV, typename S>
 void launch_wavesp(const void *tr, const double *nrmOwn, double *ws, int NF, int nE, const Phys &ph, cudaStream_t st) {
   long n = (long)NF * nE;
@@ -206,6 +211,7 @@ cudaError_t add_lines(KernelSet &k) {
 template <class C, typename R, typename S, bool BC, int RS, bool VISC>
 bool make_set(KernelSet &k, std::string &err) {
   k.trace = &launch_trace<C, R, S>;
+  k.import = &launch_import<C, R, S>;
   k.wavesp = &launch_wavesp<C::DIM, C::NV, S>;
   k.nLine = 0;
   cudaError_t e = add_lines<C, R, S, BC, RS, VISC>(k);
