@@ -33,6 +33,8 @@ struct KernelSet {
     // walking tiles with a stride of the grid size
     int persistent = 0, occ = 0;
   };
+  // indices in `tma` that the default choice names
+  enum : int { kTileOne = 0, kTileLine = 5, kTilePipe160 = 6, kTilePipe256 = 8, kTilePipe128 = 9, kTileSplit160 = 10, kTileSplit128 = 11 };
   static constexpr int kMaxTma = 16;
   TmaVariant tma[kMaxTma];
   int nTma = 0;

@@ -506,7 +506,7 @@ frg_status setup_tma(frg_solver *s) {
     const int nTiles = (s->nE + TE - 1) / TE;
     s->nBlkTma = std::min(nTiles, nSM * tv.occ);
   } else {
-    s->nBlkTma = L / TE;
+    s->nBlkTma = (s->nE + TE - 1) / TE;
   }
   return FRG_OK;
 }
@@ -521,6 +521,36 @@ void pick_line(frg_solver *s) {
     s->nBlk = (s->nE + s->line->TE - 1) / s->line->TE;
     if (s->line->rounds > 1 ? 3 * s->nBlk >= 4 * s->nSM : 2 * s->nBlk >= s->nSM) return;
   }
+}
+
+// The 2D inviscid update's tile shape until frg_autotune or frg_set_tile_variant
+// chooses another (the results are the same bits).  Per step of the vortex, us,
+// this choice / the one-tile kernel that was the default:
+//   mixed  P2 24x24 16.5/20.9  128x128 35/35  200x200 67/81
+//          P3 24x24 18.3/20.8  96x96 29/29    128x128 46/52  200x200 118/139
+//          P4 24x24 18.2/29.5  64x64 26/37    128x128 73/101 200x200 172/243
+//          P5 24x24 21.0/25.6  64x64 34/34    128x128 95/129
+//   FP64   P2 24x24 19.1/23.9  P3 48x48 20.8/27.5  P4 24x24 20.3/26.9  P5 24x24 21.6/24.6
+//          P3 200x200 183/199  P4 200x200 304/328  P5 128x128 183/191
+void pick_tile(frg_solver *s) {
+  const KernelSet &k = s->ks;
+  const int P = s->p.order;
+  const bool f32 = s->sstore == 4;
+  const auto blocks = [&](int v) { return (s->nE + k.tma[v].TE - 1) / k.tma[v].TE; };
+  const auto wave = [&](int v) { return s->nSM * k.tma[v].occ; };
+  const bool large = s->nE >= 25000;
+  // a mesh that one wave of the 256-thread pipe takes: its many threads make the
+  // shortest chain
+  if (blocks(KernelSet::kTilePipe256) <= wave(KernelSet::kTilePipe256)) s->tmaVar = KernelSet::kTilePipe256;
+  // FP32 with three quarters of a wave of line-kernel blocks or more (P = 4 only up
+  // to one wave: the split kernel passes it beyond)
+  else if (f32 && 4 * blocks(KernelSet::kTileLine) >= 3 * wave(KernelSet::kTileLine) && !(P == 4 && large))
+    s->tmaVar = KernelSet::kTileLine;
+  else if (f32) s->tmaVar = P == 4 ? KernelSet::kTileSplit160 : KernelSet::kTileOne;
+  else if (P == 5 && s->nE >= 12000) s->tmaVar = KernelSet::kTilePipe160;
+  else if (large && P == 3) s->tmaVar = KernelSet::kTilePipe128;
+  else if (large && P == 4) s->tmaVar = KernelSet::kTileSplit128;
+  else s->tmaVar = KernelSet::kTileOne;
 }
 
 frg_status launch_stage_args(frg_solver *s, StageArgs &a) {
@@ -800,6 +830,7 @@ frg_status frg_create(const frg_params *params, const frg_mesh *mesh, frg_solver
   if (s->ks.nTma > 0) {
     const char *env = getenv("FRG_KERNEL");
     s->useTma = !(env && std::strcmp(env, "generic") == 0);
+    pick_tile(s.get());
     if (s->useTma && (st = setup_tma(s.get()))) return st;
   }
   {

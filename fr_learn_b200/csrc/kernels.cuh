@@ -230,15 +230,35 @@ __device__ __forceinline__ R inviscid_common(const R *UL, const R *UR, const R *
   if constexpr (NV == 1) {
     return lax_friedrichs<DIM, R>(UL[0], UR[0], n, Fn, ph);
   } else if constexpr (RS == 0 || DIM == 3) {
-    return rusanov<DIM, NV, R, double>(UL, UR, n, Fn, ph);
+    return rusanov_normal<DIM, R, double>(UL, UR, n, Fn, ph);
   } else if constexpr (BC) {
-    if (code < 0) return rusanov<DIM, NV, R, double>(UL, UR, n, Fn, ph);
+    if (code < 0) return rusanov_normal<DIM, R, double>(UL, UR, n, Fn, ph);
     roe2d<R, double>(UL, UR, n, Fn, ph);
     return -1;
   } else {
     roe2d<R, double>(UL, UR, n, Fn, ph);
     return -1;
   }
+}
+
+// The jump Fn dA - disFn at a flux point (extrapolateNormalFlux, correctDivFlux):
+// Fn along the left element's normal, ext the contravariant flux extrapolated
+// along its coordinate.
+template <typename R>
+__device__ __forceinline__ R face_jump(R Fn, bool right, R dA, int side, R ext) {
+  return Fn * (right ? -dA : dA) - (side ? ext : -ext);
+}
+
+// RK update of one value (timeStepA/B, src/solver.cpp:307-385) from dj = divF /
+// detJ; base is the accumulator (first stage, Jameson form: U0).  Returns the new
+// state, and in accNew the new accumulator.
+__device__ __forceinline__ double rk_update(int flags, double dj, double base, double u0, double cb, double ca,
+                                            double &accNew) {
+  accNew = 0;
+  if (flags & SF_JAMESON) return base - ca * dj;
+  accNew = base - cb * dj;
+  if (flags & SF_LAST) return accNew;
+  return ((flags & SF_FIRST) ? base : u0) - ca * dj;
 }
 
 // LDG penalty sign: face::ldgSolution (src/face.cpp:590-598).

@@ -51,54 +51,6 @@ __device__ __forceinline__ int line_fpt(int dir, int side, int p, int q) {
   }
 }
 
-// face::rusanovFlux (src/face.cpp:289-356) with each side's flux formed along
-// the normal at once; the pressures in PR (double).  Returns the wave speed.
-template <int DIM, typename R, typename PR>
-__device__ __forceinline__ R rusanov_normal(const R *UL, const R *UR, const R *n, R *Fn, const Phys &ph) {
-  const PR g = (PR)ph.gamma;
-  R vn[2], p[2], eig[2];
-#pragma unroll
-  for (int s = 0; s < 2; s++) {
-    const R *U = s ? UR : UL;
-    const PR ir = (PR)1 / (PR)U[0];
-    PR vv = 0;
-    R m = 0;
-#pragma unroll
-    for (int d = 0; d < DIM; d++) {
-      const PR w = (PR)U[d + 1] * ir;
-      vv += w * w;
-      m += n[d] * U[d + 1];
-    }
-    const PR pr = (g - (PR)1.0) * ((PR)U[DIM + 1] - (PR)0.5 * (PR)U[0] * vv);
-    vn[s] = m * (R)ir;
-    p[s] = (R)pr;
-    eig[s] = fabs(vn[s]) + sqrt((R)fmax(g * pr * ir, (PR)0.0));
-  }
-  const R e = eig[0] > eig[1] ? eig[0] : eig[1];
-  Fn[0] = (R)0.5 * (UL[0] * vn[0] + UR[0] * vn[1] - e * (UR[0] - UL[0]));
-#pragma unroll
-  for (int d = 0; d < DIM; d++)
-    Fn[d + 1] = (R)0.5 * (UL[d + 1] * vn[0] + UR[d + 1] * vn[1] + (p[0] + p[1]) * n[d] - e * (UR[d + 1] - UL[d + 1]));
-  Fn[DIM + 1] = (R)0.5 * ((UL[DIM + 1] + p[0]) * vn[0] + (UR[DIM + 1] + p[1]) * vn[1] - e * (UR[DIM + 1] - UL[DIM + 1]));
-  return e;
-}
-
-// The common inviscid flux (face::calcInviscidFlux): Lax-Friedrichs, Rusanov,
-// or Roe on interior faces.  Negative return: no wave speed is kept (Roe).
-template <class C, typename R, bool BC, int RS>
-__device__ __forceinline__ R line_common(const R *UL, const R *UR, const R *n, int code, R *Fn, const Phys &ph) {
-  if constexpr (C::NV == 1) {
-    return lax_friedrichs<C::DIM, R>(UL[0], UR[0], n, Fn, ph);
-  } else {
-    if constexpr (RS == 1 && C::DIM == 2)
-      if (!BC || code >= 0) {
-        roe2d<R, double>(UL, UR, n, Fn, ph);
-        return -1;
-      }
-    return rusanov_normal<C::DIM, R, double>(UL, UR, n, Fn, ph);
-  }
-}
-
 // What one end of a line reads: the face's normal (of its left element), area,
 // neighbour code and this element's own trace; then the other side's trace.
 // The viscous stage also reads both sides' projected viscous fluxes (vo this
@@ -208,7 +160,7 @@ __device__ __forceinline__ void line_end_jump(const StageArgs &a, const LineEnd<
     UL[v] = right ? L.oth[v] : L.own[v];
     UR[v] = right ? L.own[v] : L.oth[v];
   }
-  const R ws = line_common<C, R, BC, RS>(UL, UR, L.n, L.code, Fn, a.ph);
+  const R ws = inviscid_common<C, R, BC, RS>(UL, UR, L.n, L.code, Fn, a.ph);
   const bool upd = !right && ws >= 0;
   if (a.flags & (SF_WAVESP | SF_DTNEXT)) {
     const size_t at = (size_t)L.f * a.nE + eg;
@@ -233,9 +185,8 @@ __device__ __forceinline__ void line_end_jump(const StageArgs &a, const LineEnd<
       }
     }
   }
-  const R sA = right ? -L.dA : L.dA;
 #pragma unroll
-  for (int v = 0; v < NV; v++) jump[v] = Fn[v] * sA - (side ? ext[v] : -ext[v]);
+  for (int v = 0; v < NV; v++) jump[v] = face_jump(Fn[v], right, L.dA, side, ext[v]);
 }
 
 // Both ends of a line and its part of the divergence, in place: on entry
@@ -331,18 +282,10 @@ __device__ __forceinline__ bool line_point(const StageArgs &a, int r, int e0, in
 template <class C, typename R, typename S>
 __device__ __forceinline__ R line_rk_update(const StageArgs &a, R acc, R idet, double base, double u0, size_t gi,
                                             double cb, double ca, bool check) {
-  const bool first = a.flags & SF_FIRST, last = a.flags & SF_LAST;
-  const double dj = (double)(acc * idet);  // divF / detJ
-  double unew;
-  if (a.flags & SF_JAMESON) {
-    unew = base - ca * dj;
-  } else {
-    unew = base - cb * dj;
-    if (!last) {
-      a.Acc[gi] = unew;
-      unew = (first ? base : u0) - ca * dj;
-    }
-  }
+  const bool last = a.flags & SF_LAST;
+  double accNew;
+  const double unew = rk_update(a.flags, (double)(acc * idet), base, u0, cb, ca, accNew);  // acc / detJ
+  if (!last && !(a.flags & SF_JAMESON)) a.Acc[gi] = accNew;
   if (last) {
     a.Uout[gi] = unew;
     if (check && isnan(unew)) atomicOr(a.err, ERRF_NAN);

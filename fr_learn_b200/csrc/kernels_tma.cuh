@@ -282,14 +282,14 @@ __device__ __forceinline__ void tma_phase_b(const StageArgs &a, const OpTab<R> &
     if (eg >= a.nEle) continue;
     int dir, side, s0, st;
     fpt_line<C>(f, dir, side, s0, st);
-    R own[NV], dis[NV];
+    R own[NV], ext[NV];
 #pragma unroll
     for (int v = 0; v < NV; v++) {
       R q = 0;
 #pragma unroll
       for (int j = 0; j < N1; j++) q += op.lag[side][j] * b.Fs[((dir * NV + v) * NS + s0 + j * st) * TE + e];
       own[v] = (R)b.Tw[(v * NF + f) * TE + e];
-      dis[v] = side ? q : -q;
+      ext[v] = q;
     }
     R n[DIM];
 #pragma unroll
@@ -329,10 +329,7 @@ __device__ __forceinline__ void tma_phase_b(const StageArgs &a, const OpTab<R> &
                               : (upd ? (double)ws : a.waveSp[(size_t)f * L + eg]) * a.wsurf[f % C::NFF] *
                                     a.dAd[(size_t)f * L + eg];
 #pragma unroll
-    for (int v = 0; v < NV; v++) {
-      const R fo = right ? -Fn[v] * dA : Fn[v] * dA;
-      b.Js[(v * NF + f) * TE + e] = fo - dis[v];
-    }
+    for (int v = 0; v < NV; v++) b.Js[(v * NF + f) * TE + e] = face_jump(Fn[v], right, dA, side, ext[v]);
   }
 }
 
@@ -389,29 +386,18 @@ __device__ __forceinline__ void tma_phase_c(const StageArgs &a, const OpTab<R> &
 #pragma unroll
     for (int j = 0; j < N1; j++) {
       const int s = j * N1 + i, o = (v * NS + s) * TE + e;
-      R acc = b.Us[o];
+      R acc = 0;
 #pragma unroll
       for (int q = 0; q < N1; q++) acc += op.dlag[j][q] * F[q];
       acc += -op.gL[j] * JB;
       acc += op.gR[j] * JT;
+      acc = b.Us[o] + acc;
       if (flags & SF_DIVF) a.divF[((size_t)v * NS + s) * a.ldU + eg] = (double)acc;
-      const double dj = (double)(acc * (R)b.Det[s * TE + e]);  // divF / detJ
-      double unew;
-      if (jam) {
-        unew = b.U0[o] - ca * dj;
-        if (last) b.U0[o] = unew;
-      } else {
-        const double t = cb * dj;
-        const double base = first ? b.U0[o] : b.Acc[o];
-        if (last) {
-          unew = base - t;
-          b.U0[o] = unew;
-        } else {
-          b.Acc[o] = base - t;
-          const double u0 = first ? base : b.U0[o];
-          unew = u0 - ca * dj;
-        }
-      }
+      double accNew;
+      const double unew = rk_update(flags, (double)(acc * (R)b.Det[s * TE + e]),  // divF / detJ
+                                    first || jam ? b.U0[o] : b.Acc[o], b.U0[o], cb, ca, accNew);
+      if (last) b.U0[o] = unew;
+      else if (!jam) b.Acc[o] = accNew;
       if (last && (v == 0 || v == NV - 1) && isnan(unew)) atomicOr(a.err, ERRF_NAN);
       const R un = (R)(last ? unew : (double)(S)unew);
       b.Us[o] = un;

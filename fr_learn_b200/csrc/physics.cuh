@@ -99,6 +99,38 @@ __device__ __forceinline__ R rusanov(const R *UL, const R *UR, const R *n, R *Fn
   return eig;
 }
 
+// face::rusanovFlux (src/face.cpp:289-356) with each side's flux formed along
+// the normal at once; the pressures in PR (double).  Returns the wave speed.
+template <int DIM, typename R, typename PR>
+__device__ __forceinline__ R rusanov_normal(const R *UL, const R *UR, const R *n, R *Fn, const Phys &ph) {
+  const PR g = (PR)ph.gamma;
+  R vn[2], p[2], eig[2];
+#pragma unroll
+  for (int s = 0; s < 2; s++) {
+    const R *U = s ? UR : UL;
+    const PR ir = (PR)1 / (PR)U[0];
+    PR vv = 0;
+    R m = 0;
+#pragma unroll
+    for (int d = 0; d < DIM; d++) {
+      const PR w = (PR)U[d + 1] * ir;
+      vv += w * w;
+      m += n[d] * U[d + 1];
+    }
+    const PR pr = (g - (PR)1.0) * ((PR)U[DIM + 1] - (PR)0.5 * (PR)U[0] * vv);
+    vn[s] = m * (R)ir;
+    p[s] = (R)pr;
+    eig[s] = fabs(vn[s]) + sqrt((R)fmax(g * pr * ir, (PR)0.0));
+  }
+  const R e = eig[0] > eig[1] ? eig[0] : eig[1];
+  Fn[0] = (R)0.5 * (UL[0] * vn[0] + UR[0] * vn[1] - e * (UR[0] - UL[0]));
+#pragma unroll
+  for (int d = 0; d < DIM; d++)
+    Fn[d + 1] = (R)0.5 * (UL[d + 1] * vn[0] + UR[d + 1] * vn[1] + (p[0] + p[1]) * n[d] - e * (UR[d + 1] - UL[d + 1]));
+  Fn[DIM + 1] = (R)0.5 * ((UL[DIM + 1] + p[0]) * vn[0] + (UR[DIM + 1] + p[1]) * vn[1] - e * (UR[DIM + 1] - UL[DIM + 1]));
+  return e;
+}
+
 // face::roeFlux with the entropy fix, 2D (src/face.cpp:358-484).
 template <typename R, typename PR>
 __device__ __forceinline__ void roe2d(const R *UL, const R *UR, const R *n, R *Fn, const Phys &ph) {

@@ -163,6 +163,26 @@ cudaError_t add_line(KernelSet &k) {
     return prepare_kernel(fr_line_stage_kernel<C, R, S, BC, RS, TE, NT, MB>, T::SMEM);
   }
 }
+// The line kernel among the tile shapes of the 2D inviscid update (it takes no
+// tensor maps).
+template <class C, typename R, typename S, bool BC, int RS, int TE, int NT, int MB>
+void launch_line_tile(const void *args, const void *, int nBlk, size_t smem, cudaStream_t st) {
+  launch_line(fr_line_stage_kernel<C, R, S, BC, RS, TE, NT, MB>, *static_cast<const StageArgs *>(args), nBlk, NT, smem,
+              st);
+}
+template <class C, typename R, typename S, bool BC, int RS, int TE, int NT, int MB>
+cudaError_t add_line_tile(KernelSet &k) {
+  if (k.nTma >= KernelSet::kMaxTma) return cudaErrorInvalidValue;  // the variant table is full
+  using T = LineT<C, R, TE, NT>;
+  KernelSet::TmaVariant &v = k.tma[k.nTma++];
+  v.launch = &launch_line_tile<C, R, S, BC, RS, TE, NT, MB>;
+  v.TE = TE;
+  v.NT = NT;
+  v.smem = T::SMEM;
+  auto f = fr_line_stage_kernel<C, R, S, BC, RS, TE, NT, MB>;
+  const cudaError_t e = prepare_kernel(f, T::SMEM);
+  return e == cudaSuccess ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v.occ, f, NT, T::SMEM) : e;
+}
 // Block shapes of a configuration (elements and threads per block, resident
 // blocks per SM), in the order pick_line tries them.  The first is for meshes that
 // fill the GPU several times: elements as many as keep a warp's accesses whole
@@ -222,14 +242,20 @@ bool make_set(KernelSet &k, std::string &err) {
     e = cudaFuncGetAttributes(&fa, fr_trace_kernel<C, R, S>);
   }
   if constexpr (C::DIM == 2 && !VISC) {
-    // variant 0 is the default; the others are candidates for frg_autotune
+    // the shapes frg_autotune tries and pick_tile chooses from, in the order of
+    // KernelSet's tile names
     k.nTma = 0;
     if (e == cudaSuccess) e = add_tma_variant<C, R, S, BC, RS, 0, 128>(k);
     if (e == cudaSuccess) e = add_tma_variant<C, R, S, BC, RS, 0, 256>(k);
     if (e == cudaSuccess) e = add_tma_variant<C, R, S, BC, RS, -1, 128>(k);
     if (e == cudaSuccess) e = add_tma_variant<C, R, S, BC, RS, -1, 64>(k);
     if (e == cudaSuccess) e = add_tma_variant<C, R, S, BC, RS, -2, 64>(k);
-    if (e == cudaSuccess) e = add_tma_variant<C, R, S, BC, RS, -2, 32>(k);
+    // a thread per line, loads straight to registers: FP32 a thread for every
+    // line of 32 elements, FP64 half as many
+    constexpr int n = 2 * C::N1;
+    constexpr bool f32 = sizeof(R) == 4;
+    constexpr int NT = f32 ? 32 * n : 16 * n, MB = f32 ? (C::P < 4 ? 1024 : 768) / NT : 384 / NT;
+    if (e == cudaSuccess) e = add_line_tile<C, R, S, BC, RS, 32, NT, (MB > 1 ? MB : 1)>(k);
     // persistent, ring-buffered variants
     if (e == cudaSuccess) e = add_pipe_variant<C, R, S, BC, RS, 0, 160, 2>(k);
     if (e == cudaSuccess) e = add_pipe_variant<C, R, S, BC, RS, 0, 160, 3>(k);

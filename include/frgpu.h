@@ -300,7 +300,8 @@ frg_status frg_time_stages(frg_solver *s, int nsteps, void *flush, unsigned long
 frg_status frg_autotune(frg_solver *s, int nsteps, int *variant_out, double *ms_out);
 /* Number of tile shapes the handle's configuration offers (1 without TMA). */
 frg_status frg_tile_variant_count(const frg_solver *s, int *count);
-/* Selects a tile shape of the TMA stage kernel by index (0 = default). */
+/* Selects a tile shape of the 2D stage kernel by index, in place of the one
+ * chosen for the mesh's size. */
 frg_status frg_set_tile_variant(frg_solver *s, int variant);
 /* ---- Ensemble mode (no counterpart in the reference) ---------------------
  * Many independent cases of one order in one handle: the mesh is the union
