@@ -62,9 +62,9 @@ struct LineEnd {
   R vo[VISC ? C::NV : 1], vx[VISC ? C::NV : 1], vl[VISC ? C::NV : 1];
   int f, code;
 };
-// In three steps, so that the loads of both ends and of the points are in flight
-// together: the code, what lies at the flux point itself, and the gather (of
-// the own values at a boundary, so it needs no branch).
+// In three steps, so that both ends' loads are in flight together: the code,
+// what lies at the flux point itself, and the gather (of the own values at a
+// boundary, so it needs no branch).
 template <class C, typename R, bool VISC>
 __device__ __forceinline__ void line_end_code(const StageArgs &a, LineEnd<C, R, VISC> &L, int f, int eg) {
   L.f = f;
@@ -110,20 +110,19 @@ __device__ __forceinline__ void line_end_gather(const StageArgs &a, LineEnd<C, R
     }
   }
 }
-// Both ends of a thread's line.
-template <class C, typename R, typename S, bool VISC, class LT>
-__device__ __forceinline__ void line_ends_code(const StageArgs &a, LineEnd<C, R, VISC> *E, const LT &t) {
-  if (!t.act) return;
-  line_end_code<C, R>(a, E[0], t.fpt(0), t.eg);
-  line_end_code<C, R>(a, E[1], t.fpt(1), t.eg);
-}
+// Both ends of a thread's line, in flight together.  Issued where they are used:
+// ahead of the point-wise phase, steps were 1-6 % slower at P >= 2 (2D NS 75x48 P = 4
+// FP64 86.0 against 82.5 us) and 2-4 % faster at P = 1, and 5-28 % slower where a block
+// takes its lines in rounds: the registers they hold cost more than the latency
+// they hide.
 template <class C, typename R, typename S, bool VISC, class LT>
 __device__ __forceinline__ void line_ends_load(const StageArgs &a, LineEnd<C, R, VISC> *E, const LT &t) {
-  if (!t.act) return;
-  line_end_own<C, R, S>(a, E[0], t.eg);
-  line_end_own<C, R, S>(a, E[1], t.eg);
-  line_end_gather<C, R, S>(a, E[0], t.eg);
-  line_end_gather<C, R, S>(a, E[1], t.eg);
+#pragma unroll
+  for (int s = 0; s < 2; s++) line_end_code<C, R>(a, E[s], t.fpt(s), t.eg);
+#pragma unroll
+  for (int s = 0; s < 2; s++) line_end_own<C, R, S>(a, E[s], t.eg);
+#pragma unroll
+  for (int s = 0; s < 2; s++) line_end_gather<C, R, S>(a, E[s], t.eg);
 }
 // Ghost state at a boundary end (in double, as other_side).
 template <class C, typename R, bool BC, bool VISC>
@@ -365,17 +364,15 @@ __device__ __forceinline__ void line_set(R *Bl, const R F[C::NV][C::N1]) {
 // the buffers hold the contravariant flux.
 template <class C, typename R, typename S, bool BC, int RS, int TE, class T, bool VISC>
 __device__ __forceinline__ void line_stage_end(const StageArgs &a, const OpTab<R> &op, R *B, double *Ws,
-                                               LineEnd<C, R, VISC> *E, int e0) {
+                                               int e0) {
   constexpr int NF = C::NF, NV = C::NV, DIM = C::DIM, N1 = C::N1, NL = T::NL;
   const bool resid = a.flags & SF_RESIDUAL;
 #pragma unroll 1
   for (int r = 0; r < T::LR; r++) {
     const LineThread<C, T> t(a, e0, r);
     if (!t.act) continue;
-    if (T::LR > 1) {
-      line_ends_code<C, R, S>(a, E, t);
-      line_ends_load<C, R, S>(a, E, t);
-    }
+    LineEnd<C, R, VISC> E[2];
+    line_ends_load<C, R, S>(a, E, t);
     R F[NV][N1];
     line_get<C, R, T>(B + t.base(), F);
     line_divergence<C, R, BC, RS, TE>(a, op, E, F, Ws, t.e, t.eg);
@@ -463,13 +460,9 @@ __global__ void __launch_bounds__(NT, MB) fr_line_stage_kernel(const StageArgs a
   R *B = reinterpret_cast<R *>(smem_raw + T::WS);     // [DIM][NV][NL][TE]
   const OpTab<R> &op = stage_op<R>(a);
   const int e0 = blockIdx.x * TE;
-  const LineThread<C, T> t0(a, e0, 0);
   pdl_launch_dependents();
   pdl_wait();
   stage_dt_reset(a);
-  // every load of the first half in flight at once
-  LineEnd<C, R> E[2];
-  if (T::LR == 1) line_ends_code<C, R, S>(a, E, t0);
   R u[T::NP][NV], G[T::NP][DIM][DIM];
 #pragma unroll
   for (int r = 0; r < T::NP; r++) {
@@ -478,7 +471,6 @@ __global__ void __launch_bounds__(NT, MB) fr_line_stage_kernel(const StageArgs a
     line_load_point<C, R, S>(a, s, e0 + e, u[r]);
     line_load_jg<C, R, S>(a, s, e0 + e, G[r]);
   }
-  if (T::LR == 1) line_ends_load<C, R, S>(a, E, t0);
   // contravariant flux at the solution points (calcInviscidFlux_spts)
 #pragma unroll
   for (int r = 0; r < T::NP; r++) {
@@ -489,7 +481,7 @@ __global__ void __launch_bounds__(NT, MB) fr_line_stage_kernel(const StageArgs a
     line_put_flux<C, R, T>(B, F, G[r], s % N1, (s / N1) % N1, DIM == 3 ? s / (N1 * N1) : 0, e);
   }
   __syncthreads();
-  line_stage_end<C, R, S, BC, RS, TE, T, false>(a, op, B, Ws, E, e0);
+  line_stage_end<C, R, S, BC, RS, TE, T, false>(a, op, B, Ws, e0);
 }
 
 // ----------------------------------------------------------------------------
@@ -605,17 +597,14 @@ __device__ __forceinline__ void line_gradient(const StageArgs &a, const OpTab<R>
 // (calcGradU_spts, correctGradU src/solver.cpp:808-879).
 template <class C, typename R, typename S, bool BC, class T>
 __device__ __forceinline__ void line_tile_gradient(const StageArgs &a, const OpTab<R> &op, R *B,
-                                                   const LineThread<C, T> &t0, int e0) {
+                                                   int e0) {
   constexpr int NV = C::NV, DIM = C::DIM, N1 = C::N1;
-  LineEnd<C, R> E[2];
-  if (T::LR == 1) line_ends_code<C, R, S>(a, E, t0);
   R u[T::NP][NV];
 #pragma unroll
   for (int r = 0; r < T::NP; r++) {
     int s, e;
     if (line_point<T, C::NS>(a, r, e0, s, e)) line_load_point<C, R, S>(a, s, e0 + e, u[r]);
   }
-  if (T::LR == 1) line_ends_load<C, R, S>(a, E, t0);
 #pragma unroll
   for (int r = 0; r < T::NP; r++) {
     int s, e;
@@ -627,10 +616,8 @@ __device__ __forceinline__ void line_tile_gradient(const StageArgs &a, const OpT
   for (int r = 0; r < T::LR; r++) {
     const LineThread<C, T> t(a, e0, r);
     if (!t.act) continue;
-    if (T::LR > 1) {
-      line_ends_code<C, R, S>(a, E, t);
-      line_ends_load<C, R, S>(a, E, t);
-    }
+    LineEnd<C, R> E[2];
+    line_ends_load<C, R, S>(a, E, t);
     R U[NV][N1];
     line_get<C, R, T>(B + t.base(), U);
     line_gradient<C, R, BC>(a, op, E, U);
@@ -716,10 +703,9 @@ __global__ void __launch_bounds__(NT, MB) fr_line_grad_kernel(const StageArgs a)
   R *B = reinterpret_cast<R *>(smem_raw + T::WS);  // [DIM][NV][NL][TE]
   const OpTab<R> &op = stage_op<R>(a);
   const int e0 = blockIdx.x * TE;
-  const LineThread<C, T> t0(a, e0, 0);
   pdl_launch_dependents();
   pdl_wait();
-  line_tile_gradient<C, R, S, BC, T>(a, op, B, t0, e0);
+  line_tile_gradient<C, R, S, BC, T>(a, op, B, e0);
   // physical gradient in the place of the reference-space one: d/dx_d of the
   // fields in direction d's buffer (a point's slots are read and written by its
   // own thread)
@@ -786,16 +772,13 @@ __global__ void __launch_bounds__(NT, MB)
   R *B = reinterpret_cast<R *>(smem_raw + T::WS);  // [DIM][NV][NL][TE]
   const OpTab<R> &op = stage_op<R>(a);
   const int e0 = blockIdx.x * TE;
-  const LineThread<C, T> t0(a, e0, 0);
   pdl_launch_dependents();
   pdl_wait();
   stage_dt_reset(a);
-  line_tile_gradient<C, R, S, BC, T>(a, op, B, t0, e0);
+  line_tile_gradient<C, R, S, BC, T>(a, op, B, e0);
   // inviscid + viscous flux at the solution points, transformed
   // (calcInviscidFlux_spts, calcViscousFlux_spts src/solver.cpp:562-596), over
-  // the gradient; the line ends' loads go ahead of it
-  LineEnd<C, R, true> E[2];
-  if (T::LR == 1) line_ends_code<C, R, S>(a, E, t0);
+  // the gradient
 #pragma unroll
   for (int r = 0; r < T::NP; r++) {
     int s, e;
@@ -813,9 +796,8 @@ __global__ void __launch_bounds__(NT, MB)
       for (int v = 0; v < NV; v++) F[d][v] += Fv[d][v];
     line_put_flux<C, R, T>(B, F, G, i, j, k, e);
   }
-  if (T::LR == 1) line_ends_load<C, R, S>(a, E, t0);
   __syncthreads();
-  line_stage_end<C, R, S, BC, RS, TE, T, true>(a, op, B, Ws, E, e0);
+  line_stage_end<C, R, S, BC, RS, TE, T, true>(a, op, B, Ws, e0);
 }
 
 }  // namespace frg
