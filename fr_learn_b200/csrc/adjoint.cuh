@@ -16,9 +16,9 @@
 //   fbar[f]      = +-dA Jbar[f] from this element's copy of the common flux
 //                  plus the neighbour's copy (both elements evaluate the same
 //                  face flux), gathered from the face-seed pass
-//   Ubar_f       = (dFn/dU_own)^T fbar   (dual numbers; on boundaries the
-//                  ghost state is differentiated with the interior state, and
-//                  the freestream-parameter column gives dJ/dtheta)
+//   Ubar_f       = (dFn/dU_own)^T fbar   (reverse-mode products; on boundaries
+//                  the ghost state is differentiated with the interior state,
+//                  and the freestream parameter's component gives dJ/dtheta)
 //   Fsbar_d[s]   = sum_i dlag[i][c_d(s)] gbar[line pt i] - sum_f (+-) lag Jbar[f]
 //   Ubar[s]      = sum_d (dF_d/dU)^T (sum_d1 JGinv[d1][d] Fsbar_d1) + sum_f lag Ubar_f
 //
