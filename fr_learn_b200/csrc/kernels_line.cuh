@@ -14,13 +14,13 @@
 // instruction issue (every output re-read its lines from shared memory and
 // indexed the operators by thread).  Here it is the latency of the loads, which
 // are plain coalesced loads (element index fastest): long-scoreboard stalls are
-// 6.7 of the 18 cycles a warp spends per instruction, DRAM is at 35 %.  Per step,
+// 4.4 of the 15.8 cycles a warp spends per instruction (barriers 1.9), DRAM is at 35 %.  Per step,
 // us, before and after (one B200):
 //   3D Euler 31x29x27   P = 3 FP32 1184 -> 572   FP64 1684 -> 882
 //   3D Euler 16x16x16   P = 3 FP32  172 ->  97   FP64  300 -> 180
 //   3D NS    32x32x32   P = 3 FP32 1840 -> 1471  FP64 3947 -> 3017 (before: a TMA pair)
 //   3D NS    28x28x28   P = 2 FP32  854 -> 556   FP64 2147 -> 1045
-//   2D NS    150x96     P = 3 FP32  198 -> 130;  75x48 P = 4 FP64 127 -> 94
+//   2D NS    150x96     P = 3 FP32  198 -> 117;  75x48 P = 4 FP64 127 -> 82.5
 // Tried and not kept: a thread per column of an element that takes the three
 // directions in turn, its own column in registers (573 on the first line, twice
 // the latency on small meshes); L2 prefetch of the next wave's tile (5-12 %
