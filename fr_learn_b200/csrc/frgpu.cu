@@ -1492,6 +1492,40 @@ frg_status frg_update(frg_solver *s, int nsteps) {
   return check_flags(s);
 }
 
+// Where a kernel may store `bytes` in the place of a copy to `host`: the device's
+// address of `host` if all of those bytes lie in the one pinned range [start, start
+// + size) that the driver names for it, the device may write there (memory can be
+// registered read-only) and a double is aligned; else null.  memType and access are
+// the driver's CU_POINTER_ATTRIBUTE_MEMORY_TYPE and _ACCESS_FLAGS of `host`.
+void *frg_direct_target(const void *host, unsigned long long bytes, unsigned memType, unsigned access,
+                        unsigned long long dev, unsigned long long start, unsigned long long size) {
+  const unsigned long long h = reinterpret_cast<unsigned long long>(host);
+  if (memType != CU_MEMORYTYPE_HOST || access != CU_POINTER_ATTRIBUTE_ACCESS_FLAG_READWRITE || !dev) return nullptr;
+  if (h % alignof(double) || dev % alignof(double) || h < start || bytes > size || h - start > size - bytes)
+    return nullptr;
+  return reinterpret_cast<void *>(dev);
+}
+static double *direct_target(const double *host, size_t bytes) {
+  typedef CUresult (*Fn)(unsigned, CUpointer_attribute *, void **, CUdeviceptr);
+  static Fn fn = nullptr;
+  static std::once_flag once;
+  std::call_once(once, [] {
+    void *p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuPointerGetAttributes", &p, cudaEnableDefault, &q) == cudaSuccess &&
+        q == cudaDriverEntryPointSuccess)
+      fn = reinterpret_cast<Fn>(p);
+  });
+  unsigned type = 0, access = 0;
+  CUdeviceptr dev = 0, start = 0;
+  size_t size = 0;
+  CUpointer_attribute at[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_ACCESS_FLAGS,
+                              CU_POINTER_ATTRIBUTE_DEVICE_POINTER, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
+                              CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+  void *out[] = {&type, &access, &dev, &start, &size};
+  if (!fn || fn(5, at, out, (CUdeviceptr)host) != CUDA_SUCCESS) return nullptr;
+  return static_cast<double *>(frg_direct_target(host, bytes, type, access, dev, start, size));
+}
 constexpr size_t kDirectBytes = size_t(256) << 10;
 // Upload, steps, download and the flag word on the handle's stream with one
 // synchronisation at the end (the host waits once per call, not after each
@@ -1519,11 +1553,7 @@ frg_status frg_update_host(frg_solver *s, double *U_host, int nsteps) {
   // the flag word goes to the host with the state; a small state goes straight
   // into the caller's buffer where that is pinned (the copy's own latency, about
   // 5 us, is more than its bytes take: below kDirectBytes)
-  double *direct = nullptr;
-  cudaPointerAttributes at;
-  if (n * 8 <= kDirectBytes && cudaPointerGetAttributes(&at, U_host) == cudaSuccess && at.type == cudaMemoryTypeHost)
-    direct = static_cast<double *>(at.devicePointer);
-  cudaGetLastError();  // (an unknown pointer is no error)
+  double *const direct = n * 8 <= kDirectBytes ? direct_target(U_host, n * 8) : nullptr;
   to_ref_layout(s, s->U, direct ? direct : s->scratchRef, s->nS, s->hostFlag);
   if ((st = post_launch(s))) return st;
   if (!direct) CK(cudaMemcpyAsync(U_host, s->scratchRef, n * 8, cudaMemcpyDeviceToHost, s->stream));
