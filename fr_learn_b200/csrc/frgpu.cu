@@ -427,6 +427,7 @@ StageArgs base_args(frg_solver *s) {
   a.grp = s->grp;
   a.dtLocal = s->p.dtType == 2;
   a.time = s->timeDev;
+  a.dtTime = dt_slot(s, s->dtCur);
   a.err = s->err;
   a.vcjh = s->p.vcjhScheme;
   a.ph = make_phys(s->p);

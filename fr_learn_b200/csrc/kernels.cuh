@@ -156,6 +156,7 @@ struct StageArgs {
   const double *dt;     // scalar, [nE] when dtLocal, or one per group when grp is set
   const int *grp;       // ensemble mode: group (independent case) of each element, else null
   double *time;         // device time (SF_TIME)
+  const double *dtTime; // what it advances by: the global dt, with dtLocal the smallest of the elements'
   unsigned *err;
   double aNext, bCur;
   int dtLocal, flags, vcjh;

@@ -424,7 +424,7 @@ __device__ __forceinline__ void line_stage_end(const StageArgs &a, const OpTab<R
     }
   }
   if (resid) return;
-  if ((a.flags & SF_TIME) && !a.grp && blockIdx.x == 0 && threadIdx.x == 0) *a.time += stage_dt(a);
+  if ((a.flags & SF_TIME) && !a.grp && blockIdx.x == 0 && threadIdx.x == 0) stage_time(a, stage_dt(a));
   __syncthreads();
 #pragma unroll 1
   for (int r = 0; r < T::LR; r++) {

@@ -111,6 +111,13 @@ __device__ __forceinline__ double stage_dt(const StageArgs &a) {
   return x;
 }
 
+// The step's end: params->time += params->dt (solver::update).  With local time
+// steps params->dt is the smallest of the elements' (calcDt, src/solver.cpp:293-305),
+// which the dt kernel left before the stages; dtG is the global dt otherwise.
+__device__ __forceinline__ void stage_time(const StageArgs &a, double dtG) {
+  *a.time += a.dtLocal ? __ldcg(a.dtTime) : dtG;
+}
+
 // First stage of a step with the fused dt: the slot the last stage will
 // minimise the next dt into starts at a huge value (the bytes 0x7F, as a
 // memset before the step would leave it); the stages in between do not read it.
@@ -538,7 +545,7 @@ __global__ void __launch_bounds__(NTV, (TileT<C, R, S, TEV, NTV>::MINB))
 
   // ---- phase C: divergence + correction, RK update into the staging tiles
   tma_phase_c<C, R, S, TE, NT>(a, op, b, e0, dtG);
-  if ((flags & SF_TIME) && !a.grp && blockIdx.x == 0 && tid == 0) *a.time += dtG;
+  if ((flags & SF_TIME) && !a.grp && blockIdx.x == 0 && tid == 0) stage_time(a, dtG);
   fence_proxy_async();
   __syncthreads();
   if (tid == 0) {
@@ -758,7 +765,7 @@ __global__ void __launch_bounds__(NT, (PipeT<C, R, S, TEV, NT, NB>::MINB))
     if (tid == 0) tma_wait_reads();
     return;
   }
-  if ((flags & SF_TIME) && !a.grp && blockIdx.x == 0 && tid == 0) *a.time += dtG;
+  if ((flags & SF_TIME) && !a.grp && blockIdx.x == 0 && tid == 0) stage_time(a, dtG);
   if (dtn && (tid >> 5) == NT / 32 - 1) {
     if (prevE0 >= 0) dtMin = fmin(dtMin, tma_tile_dt<NF, TE>(a, slot(0).Ws, prevE0, tid & 31));
     tma_dt_reduce(a, dtMin);
@@ -1029,7 +1036,7 @@ __global__ void __launch_bounds__(NT, (SplitT<C, R, S, TEV, NT>::MINB))
     if (tid == 0) tma_wait_reads();
     return;
   }
-  if ((flags & SF_TIME) && !a.grp && blockIdx.x == 0 && tid == 0) *a.time += dtG;
+  if ((flags & SF_TIME) && !a.grp && blockIdx.x == 0 && tid == 0) stage_time(a, dtG);
   if (dtn && (tid >> 5) == NT / 32 - 1) {
     if (prevE0 >= 0)
       dtMin = fmin(dtMin, tma_tile_dt<NF, TE>(a, slot(0).Ws, prevE0, tid & 31, &volB[((j - 1) & 1) * TE]));
