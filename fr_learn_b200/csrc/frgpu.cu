@@ -98,11 +98,12 @@ __global__ void __launch_bounds__(256) fr_dt_kernel(const double *__restrict__ w
 
 // Ensemble mode, once per step before the stages: each group's time advances
 // by the dt its elements use this step, and the slot the last stage
-// minimises the next dt into is reset.
-__global__ void fr_group_step_kernel(const double *dtCur, double *dtNext, double *time, int nGrp) {
+// minimises the next dt into is reset.  err: if not null, the step's dt is checked.
+__global__ void fr_group_step_kernel(const double *dtCur, double *dtNext, double *time, int nGrp, unsigned *err) {
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= nGrp) return;
   time[g] += dtCur[g];
+  if (err && !(dtCur[g] >= 1e-13)) atomicOr(err, ERRF_DT);
   if (dtNext) dtNext[g] = __longlong_as_double(0x7f7f7f7f7f7f7f7fLL);
 }
 
@@ -412,6 +413,10 @@ double *dt_slot(frg_solver *s, int slot) {
   return s->grp ? s->grpDt + (size_t)slot * s->nGrp : s->dtDev + slot;
 }
 
+// the elements' own dt, in one array or (dt_used) in one per dt slot
+bool dt_used(const frg_solver *s);
+double *ele_dt(frg_solver *s, int slot) { return s->eleDt + (dt_used(s) ? (size_t)slot * s->L : 0); }
+
 StageArgs base_args(frg_solver *s) {
   StageArgs a{};
   a.nE = s->L;
@@ -423,7 +428,7 @@ StageArgs base_args(frg_solver *s) {
   a.JG = s->JG;
   a.invDet = s->invDetS;
   a.waveSp = s->waveSp;
-  a.dt = s->p.dtType == 2 ? s->eleDt : dt_slot(s, s->dtCur);
+  a.dt = s->p.dtType == 2 ? ele_dt(s, s->dtCur) : dt_slot(s, s->dtCur);
   a.grp = s->grp;
   a.dtLocal = s->p.dtType == 2;
   a.time = s->timeDev;
@@ -441,7 +446,7 @@ StageArgs base_args(frg_solver *s) {
   a.wsurf = s->wsurf;
   a.blockMin = s->blockMin;
   a.dtNext = dt_slot(s, s->dtCur ^ 1);
-  a.eleDt = s->eleDt;
+  a.eleDt = ele_dt(s, s->dtCur ^ 1);
   a.ticket = s->ticket;
   a.cflFac = s->p.CFL * kCflLimit[s->p.order] * 2;
   a.nff = s->g.nFF;
@@ -573,7 +578,8 @@ frg_status launch_dt(frg_solver *s) {
   double fac = s->p.CFL * kCflLimit[s->p.order] * 2;
   if (s->grp) CK(cudaMemsetAsync(dt_slot(s, s->dtCur), 0x7F, (size_t)s->nGrp * 8, s->stream));
   fr_dt_kernel<<<nb, 256, 0, s->stream>>>(s->waveSp, s->dAd, s->vol, s->wsurf, s->nF, s->g.nFF, s->nE, s->L, fac,
-                                           s->eleDt, s->blockMin, s->ticket, dt_slot(s, s->dtCur), s->err, s->grp);
+                                           ele_dt(s, s->dtCur), s->blockMin, s->ticket, dt_slot(s, s->dtCur), s->err,
+                                           s->grp);
   s->dtLast = s->dtCur;
   return post_launch(s);
 }
@@ -605,8 +611,17 @@ bool fused_dt(const frg_solver *s) { return s->p.dtType == 1; }
 
 frg_status launch_group_step(frg_solver *s) {
   fr_group_step_kernel<<<(s->nGrp + 127) / 128, 128, 0, s->stream>>>(
-      dt_slot(s, s->dtCur), fused_dt(s) ? dt_slot(s, s->dtCur ^ 1) : nullptr, s->grpTime, s->nGrp);
+      dt_slot(s, s->dtCur), fused_dt(s) ? dt_slot(s, s->dtCur ^ 1) : nullptr, s->grpTime, s->nGrp,
+      dt_used(s) ? s->err : nullptr);
   return post_launch(s);
+}
+
+// Everywhere but in the 2D tile shapes what a call shows of dt is the last step's,
+// although the next one is there already: its check (SF_DTUSED), the elements' dt
+// and the dt of frg_time_step_a/b.
+bool dt_used(const frg_solver *s) { return fused_dt(s) && !s->useTma; }
+const double *manual_dt(const frg_solver *s) {
+  return s->p.dtType == 2 ? s->eleDt : s->dtDev + (dt_used(s) ? s->dtLast : s->dtCur);
 }
 
 // dt work at the start of the next fused step (see frg_solver::graph).
@@ -656,7 +671,7 @@ frg_status enqueue_step(frg_solver *s, int mode, cudaEvent_t *ev = nullptr, bool
       a.flags |= SF_DIVF;
       a.divF = s->divF[0];
     }
-    if (last && fused_dt(s)) a.flags |= SF_DTNEXT;
+    if (last && fused_dt(s)) a.flags |= SF_DTNEXT | (dt_used(s) ? SF_DTUSED : 0);
     if (first) a.dtReset = dtReset;
     // stages that follow a stage kernel directly: programmatic dependent launch
     // (not when each launch is timed on its own)
@@ -817,7 +832,7 @@ frg_status frg_create(const frg_params *params, const frg_mesh *mesh, frg_solver
     CK(cudaMemcpy(s->nbr, nb.data(), nb.size() * sizeof(int), cudaMemcpyHostToDevice));
   }
   const int nbDt = (s->nE + 31) / 32;
-  if ((st = dalloc(&s->waveSp, (size_t)s->nF * s->L)) || (st = dalloc(&s->eleDt, (size_t)s->L)) ||
+  if ((st = dalloc(&s->waveSp, (size_t)s->nF * s->L)) || (st = dalloc(&s->eleDt, 2 * (size_t)s->L)) ||
       (st = dalloc(&s->dtDev, 2)) || (st = dalloc(&s->timeDev, 1)) || (st = dalloc(&s->blockMin, (size_t)s->L)) ||
       (st = dalloc(&s->normPartial, (size_t)nbDt * s->nV)) || (st = dalloc(&s->normOut, (size_t)s->nV)) ||
       (st = dalloc(&s->err, 1)) || (st = dalloc(&s->ticket, 1)))
@@ -1173,7 +1188,7 @@ frg_status frg_download(frg_solver *s, int array, int stage, double *host) {
       return FRG_OK;
     }
     case FRG_ELE_DT:
-      CK(cudaMemcpyAsync(host, s->eleDt, (size_t)s->nE * 8, cudaMemcpyDeviceToHost, s->stream));
+      CK(cudaMemcpyAsync(host, ele_dt(s, s->dtLast), (size_t)s->nE * 8, cudaMemcpyDeviceToHost, s->stream));
       CK(cudaStreamSynchronize(s->stream));
       return FRG_OK;
     default:
@@ -1302,7 +1317,7 @@ frg_status frg_time_step_a(frg_solver *s, int step, double rkval) {
   if (s->grp) return fail(FRG_ERR_ARG, "ensemble mode: advance with frg_update");
   const long n = (long)s->nV * s->nS * s->L;
   fr_timestep_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s->stream>>>(
-      s->U, s->U0, s->divF[step], s->detJd, s->p.dtType == 2 ? s->eleDt : s->dtDev + s->dtCur, s->p.dtType == 2, rkval, 0,
+      s->U, s->U0, s->divF[step], s->detJd, manual_dt(s), s->p.dtType == 2, rkval, 0,
       s->nS, s->nE, s->L, n);
   s->trValid = false;
   return post_launch(s);
@@ -1313,7 +1328,7 @@ frg_status frg_time_step_b(frg_solver *s, int step) {
   if (s->grp) return fail(FRG_ERR_ARG, "ensemble mode: advance with frg_update");
   const long n = (long)s->nV * s->nS * s->L;
   fr_timestep_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s->stream>>>(
-      s->U, s->U0, s->divF[step], s->detJd, s->p.dtType == 2 ? s->eleDt : s->dtDev + s->dtCur, s->p.dtType == 2,
+      s->U, s->U0, s->divF[step], s->detJd, manual_dt(s), s->p.dtType == 2,
       s->RKb[step], 1, s->nS, s->nE, s->L, n);
   s->trValid = false;
   return post_launch(s);

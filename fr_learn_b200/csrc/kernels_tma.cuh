@@ -116,6 +116,7 @@ __device__ __forceinline__ double stage_dt(const StageArgs &a) {
 // which the dt kernel left before the stages; dtG is the global dt otherwise.
 __device__ __forceinline__ void stage_time(const StageArgs &a, double dtG) {
   *a.time += a.dtLocal ? __ldcg(a.dtTime) : dtG;
+  if ((a.flags & SF_DTUSED) && !(dtG >= 1e-13)) atomicOr(a.err, ERRF_DT);
 }
 
 // First stage of a step with the fused dt: the slot the last stage will
@@ -445,6 +446,18 @@ __device__ __forceinline__ void tma_phase_d(const OpTab<R> &op, const R *Us, S *
   }
 }
 
+// One dt into the minimum of a slot that was set to a huge value: a 64-bit atomicMin on the bit
+// pattern (positive doubles order like their bit patterns).  The check of dt
+// (writeResidual, src/output.cpp:823-824) is of the dt a step has used: with
+// SF_DTUSED it is made there, and a NaN, which the minimum would pass over, gets
+// there as 0.  The 2D tile shapes make it here, a step ahead.
+__device__ __forceinline__ void tma_dt_min(const StageArgs &a, double *slot, double dt) {
+  if (a.flags & SF_DTUSED) dt = dt > 0 ? dt : 0.0;
+  else if (!(dt > 1e-13)) atomicOr(a.err, ERRF_DT);  // also catches NaN
+  if (dt > 0 || (a.flags & SF_DTUSED))  // a tiny dt is still used, as the reference does before its check
+    atomicMin(reinterpret_cast<unsigned long long *>(slot), (unsigned long long)__double_as_longlong(dt));
+}
+
 // ele::calcDt for element e0 + ln (lane ln < TE) with the wave speeds this stage
 // left (src/ele.cpp:1086-1105; flux points summed in order).  Returns the
 // element's dt (INFINITY for other threads); in ensemble mode also reduces
@@ -459,28 +472,17 @@ __device__ __forceinline__ double tma_tile_dt(const StageArgs &a, const double *
   for (int f = 0; f < NF; f++) iw += Ws[f * TE + ln];
   const double dte = a.cflFac * (volS ? volS[ln] : a.vol[eg]) / iw;
   a.eleDt[eg] = dte;
-  if (a.grp) {  // ensemble mode: each element into its own group's minimum
-    if (!(dte > 1e-13)) atomicOr(a.err, ERRF_DT);
-    if (dte > 0)  // a tiny dt is still used, as the reference does before its check
-      atomicMin(reinterpret_cast<unsigned long long *>(a.dtNext + a.grp[eg]),
-                (unsigned long long)__double_as_longlong(dte));
-  }
+  if (a.grp) tma_dt_min(a, a.dtNext + a.grp[eg], dte);  // ensemble mode: each element into its own group's minimum
   return dte;
 }
 
-// Warp 0: minimum of the lanes' dt, then the global minimum by a 64-bit
-// atomicMin on the bit pattern (positive doubles order like their bit
-// patterns) into the next step's dt slot, which the host set to a huge value.
+// Warp 0: minimum of the lanes' dt, then the global minimum in the next step's dt slot.
 __device__ __forceinline__ void tma_dt_reduce(const StageArgs &a, double my) {
   for (int o = 16; o > 0; o >>= 1) {
     const double t = __shfl_xor_sync(0xffffffffu, my, o);
     my = (isnan(t) || t < my) ? t : my;
   }
-  if ((threadIdx.x & 31) == 0 && !a.grp) {
-    if (!(my > 1e-13)) atomicOr(a.err, ERRF_DT);  // also catches NaN
-    if (my > 0)  // a tiny dt is still used, as the reference does before its check
-      atomicMin(reinterpret_cast<unsigned long long *>(a.dtNext), (unsigned long long)__double_as_longlong(my));
-  }
+  if ((threadIdx.x & 31) == 0 && !a.grp) tma_dt_min(a, a.dtNext, my);
 }
 
 template <class C, typename R, typename S, bool BC, int RS, int TEV, int NTV>
