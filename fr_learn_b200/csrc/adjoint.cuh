@@ -458,8 +458,8 @@ __global__ void __launch_bounds__(AdjTile<C>::NT, AdjTile<C>::MINB) fr_adj_stage
   const int p = DIM == 2 ? c : c % N1, q = DIM == 2 ? 0 : c / N1;
   const bool act = eg < a.nEle && it < 2 * NLN;
   const int base = dir * T::BUF + c * T::N1P * TE + e, end = (side * NV * NLN + ln) * TE + e;
-  pdl_launch_dependents();
   pdl_wait();
+  pdl_launch_dependents();
 
   // ---- the seed's points into lines, and this thread's end
   const size_t fl = (size_t)NF * L, at = (size_t)(act ? line_fpt<C>(dir, side, p, q) : 0) * L + eg;

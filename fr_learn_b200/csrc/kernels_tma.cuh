@@ -94,8 +94,8 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // previous stage's last blocks still run; they issue the loads of the
 // read-only metric tiles, then wait (pdl_wait) until the previous grid has
 // finished and its writes are visible before touching anything a stage
-// writes.  Each block signals at its start that the next stage may be
-// scheduled (it is, once every block of this grid has signalled or exited).
+// writes.  Each block of the TMA kernels signals at its start that the next stage
+// may be scheduled (it is, once every block of this grid has signalled or exited).
 // Launched without the attribute, both are no-ops.
 __device__ __forceinline__ void pdl_launch_dependents() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
