@@ -72,8 +72,11 @@ struct AdjArgs {
   double *thetaBar;       // += fbar . dFn/dtheta over boundary flux points
   AdjViscBufs v;          // viscous runs only
   Phys ph;
-  OpTab<double> op;       // the run's 1D operators (inviscid stage kernel)
+  // (the 1D operators of the inviscid stage kernel are a parameter of its own: the
+  // viscous kernels keep a copy of this block on each thread's stack, and 560 bytes
+  // more of it took their element pass of 150x149 quads, P = 1, from 844 to 928 us)
 };
+static_assert(sizeof(AdjArgs) <= 464, "copied to each thread's stack by the viscous kernels");
 
 enum : int {
   ADJ_PLAIN = 1,      // write ybar only
@@ -437,7 +440,7 @@ struct AdjTile {
 };
 
 template <class C, bool BC, int RS>
-__global__ void __launch_bounds__(AdjTile<C>::NT, AdjTile<C>::MINB) fr_adj_stage_kernel(const AdjArgs a) {
+__global__ void __launch_bounds__(AdjTile<C>::NT, AdjTile<C>::MINB) fr_adj_stage_kernel(const AdjArgs a, const OpTab<double> op) {
   using A = AdjTile<C>;
   using T = typename A::T;
   constexpr int TE = A::TE, NT = A::NT, NS = C::NS, NF = C::NF, NV = C::NV, DIM = C::DIM, N1 = C::N1;
@@ -447,7 +450,6 @@ __global__ void __launch_bounds__(AdjTile<C>::NT, AdjTile<C>::MINB) fr_adj_stage
   double *W = G + A::BUF;                            // the traces' part of the state's adjoint
   double *JB = W + A::BUF, *UB = JB + A::ENDS;       // [side][NV][line][TE]: jump and trace adjoints at the ends
   __shared__ double red[NT / 32];
-  const OpTab<double> &op = a.op;
   const Phys &ph = a.ph;
   const int e0 = blockIdx.x * TE, L = a.nE;
   StageArgs sa{};  // the size line_point reads

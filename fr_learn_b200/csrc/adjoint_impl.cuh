@@ -22,7 +22,7 @@ void launch_adj_face(const AdjArgs &a, cudaStream_t st) {
 }
 // A reversed stage; with a.pdl a programmatic dependent of the launch before.
 template <class C, bool BC, int RS>
-void launch_adj_stage(const AdjArgs &a, cudaStream_t st) {
+void launch_adj_stage(const AdjArgs &a, const OpTab<double> &op, cudaStream_t st) {
   using T = AdjTile<C>;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((a.nEle + T::TE - 1) / T::TE);
@@ -34,7 +34,7 @@ void launch_adj_stage(const AdjArgs &a, cudaStream_t st) {
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
   cfg.numAttrs = a.pdl ? 1 : 0;
-  cudaLaunchKernelEx(&cfg, fr_adj_stage_kernel<C, BC, RS>, a);
+  cudaLaunchKernelEx(&cfg, fr_adj_stage_kernel<C, BC, RS>, a, op);
 }
 template <class C>
 void launch_entropy(const double *U, const double *detJ, const double *wvol, int nE, int L, const Phys &ph,
@@ -59,7 +59,7 @@ struct AdjGradShape {
 // Viscous residuals: the forward gradient / projected-flux pass on the stage
 // state, then the two adjoint passes.
 template <class C, bool BC, int RS>
-void launch_adjv_elem(const AdjArgs &a, cudaStream_t st) {
+void launch_adjv_elem(const AdjArgs &a, const OpTab<double> &, cudaStream_t st) {
   using TV = AdjGradShape<C>;
   StageArgs f{};
   f.nE = a.nE;

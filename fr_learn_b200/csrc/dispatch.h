@@ -57,10 +57,12 @@ struct KernelKey {
 };
 
 struct AdjArgs;
+template <typename R>
+struct OpTab;
 // The discrete-adjoint kernels of one configuration (FP64 only).
 struct AdjSet {
   void (*face)(const AdjArgs &a, cudaStream_t st) = nullptr;
-  void (*elem)(const AdjArgs &a, cudaStream_t st) = nullptr;
+  void (*elem)(const AdjArgs &a, const OpTab<double> &op, cudaStream_t st) = nullptr;
   // objectives: per-block partial sums into `part` (obj_blocks entries)
   void (*entropy)(const double *U, const double *detJ, const double *wvol, int nE, int L, const Phys &ph,
                   double *grad, double *part, cudaStream_t st) = nullptr;

@@ -1981,9 +1981,6 @@ AdjArgs adj_args(frg_solver *s, const double *Y, const double *gbar) {
   a.thetaDir = s->adj->thetaDir;
   a.grp = s->grp;
   a.dtGrp = s->grpDt;  // slot 0: the fixed per-group dt
-  StageArgs ops{};
-  set_stage_ops(ops, s->ops);
-  a.op = ops.opd;
   a.v = AdjViscBufs{s->adj->vg, s->adj->vfvn, s->adj->vfvn2, s->adj->vub, s->adj->vufb, s->adj->vdcb,
                     s->visc2 ? 1 : 0};
   a.ph = make_phys(s->p);
@@ -1998,7 +1995,9 @@ frg_status adj_launch(frg_solver *s, const AdjArgs &a, bool face = true) {
     s->adj->ks.face(a, s->stream);
     if ((st = post_launch(s))) return st;
   }
-  s->adj->ks.elem(a, s->stream);
+  StageArgs ops{};
+  set_stage_ops(ops, s->ops);
+  s->adj->ks.elem(a, ops.opd, s->stream);
   s->launches += s->adj->ks.elemLaunches - 1;
   return post_launch(s);
 }
