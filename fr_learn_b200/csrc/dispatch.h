@@ -47,7 +47,7 @@ struct KernelSet {
     int rounds = 0;  // of the line-wise phases
     size_t smem = 0;
   };
-  static constexpr int kMaxLine = 3;
+  static constexpr int kMaxLine = 4;
   LineVariant line[kMaxLine];
   int nLine = 0;
 };

@@ -518,15 +518,24 @@ frg_status setup_tma(frg_solver *s) {
 }
 
 // The line kernels' block shape for this mesh: the first that still gives every
-// other SM a block, or, where a block takes its lines in rounds, four blocks to
-// three SMs (both sides measured, see line_shape: a half-full GPU of wide tiles
-// is as fast as a full one of tiles half as wide, a quarter-full one is not).
+// other SM a block (of tiles half as wide, one wave does not hold the mesh), or,
+// where a block takes its lines in rounds, four blocks to three SMs (both sides
+// measured, see line_shape: a half-full GPU of wide tiles is as fast as a full one
+// of tiles half as wide, a quarter-full one is not).
+//
+// 3D viscous passes that one wave holds, but not two launches side by side, are
+// launched without the programmatic attribute: a launch's first blocks start on the
+// SMs that the launch before leaves free, and where two fit an SM the rest double up
+// there.  Per step, us, with / without: 448 hexes P = 3 FP32 89 / 76, 900 hexes P = 2
+// FP32 70 / 57.  On smaller grids the overlap is worth more (48 hexes P = 2 FP32 53
+// / 57), and no P = 1 or 2D mesh was slower for it.
 void pick_line(frg_solver *s) {
   for (int i = 0; i < s->ks.nLine; i++) {
     s->line = &s->ks.line[i];
     s->nBlk = (s->nE + s->line->TE - 1) / s->line->TE;
-    if (s->line->rounds > 1 ? 3 * s->nBlk >= 4 * s->nSM : 2 * s->nBlk >= s->nSM) return;
+    if (s->line->rounds > 1 ? 3 * s->nBlk >= 4 * s->nSM : 2 * s->nBlk > s->nSM) break;
   }
+  if (s->line->grad && s->p.nDims == 3 && s->p.order > 1 && s->nBlk <= s->nSM && 2 * s->nBlk > s->nSM) s->pdl = false;
 }
 
 // The 2D inviscid update's tile shape until frg_autotune or frg_set_tile_variant
@@ -841,7 +850,7 @@ frg_status frg_create(const frg_params *params, const frg_mesh *mesh, frg_solver
   if (p.dtType == 0) CK(cudaMemcpy(s->dtDev, &p.dt, sizeof(double), cudaMemcpyHostToDevice));
   {
     const char *pe = getenv("FRG_PDL");
-    s->pdl = !(pe && std::strcmp(pe, "0") == 0);
+    if (pe && std::strcmp(pe, "0") == 0) s->pdl = false;
   }
   if (s->ks.nTma > 0) {
     const char *env = getenv("FRG_KERNEL");

@@ -199,7 +199,14 @@ cudaError_t add_line_tile(KernelSet &k) {
 // SM gets one block or none (1,287 hexes, P = 2, FP64, viscous: 16 x 448: 116,
 // 16 x 224: 176), and the last is the narrowest, for meshes too small to give every
 // other SM a wider tile (216 hexes, P = 3, FP64: 4 x 192: 40, 8 x 384: 45,
-// 16 x 384: 76).
+// 16 x 384: 76).  Viscous passes on such meshes are a chain of point-wise and
+// line-wise phases, so their narrowest shapes have a thread for every point too
+// (48 / 294 hexes: P = 3 FP64 4 x 192: 80.5 / 89.1, 4 x 256: 76.0 / 83.1; FP32 71.9 /
+// 81.6, 65.3 / 74.2; P = 4 FP32 4 x 320: 100 / 112, 4 x 512: 95 / 108; FP64 4 x 320:
+// 130.7 / 142.3, 2 x 256: 108.0 / 116.1, but 448 hexes, 1.5 blocks of 2 elements to an
+// SM, 148 against 226; 900 hexes, P = 3 FP32: 16 x 768: 105, 8 x 512: 80, 4 x 256: 110).
+// P = 1 FP64, inviscid, 31,744 / 83,248 hexes: 16 x 192 x 2: 230 / 596, 32 x 192 x 2:
+// 205 / 494 (a residual 51.9 / 130, 45.8 / 110).
 struct LineShape {
   int TE, NT, MB;
 };
@@ -208,13 +215,18 @@ constexpr LineShape line_shape(int tier) {
   constexpr bool f32 = sizeof(R) == 4;
   constexpr int n = 2 * C::N1;  // 2D: lines per element
   constexpr LineShape none{0, 0, 0};
-  constexpr LineShape two[3] = {{32, 32 * n, (f32 ? 768 : 384) / (32 * n)}, {8, (8 * n + 31) & ~31, 1}, none};
-  constexpr LineShape p1[3] = {f32 ? LineShape{32, 384, 2} : LineShape{16, 192, 2}, {8, 96, 1}, none};
-  constexpr LineShape p2[3] = {f32 ? LineShape{32, 288, 2} : LineShape{16, 224, 2}, {16, 448, 1}, {8, 224, 1}};
-  constexpr LineShape p3[3] = {f32 ? LineShape{32, 768, 1} : LineShape{16, 384, 1},
-                               f32 ? LineShape{16, 768, 1} : LineShape{8, 384, 1}, {4, 192, 1}};
-  constexpr LineShape p4[3] = {f32 ? LineShape{16, 608, 1} : LineShape{8, VISC ? 608 : 320, 1}, {8, 608, 1},
-                               {4, 320, 1}};
+  using Shapes = LineShape[KernelSet::kMaxLine];
+  constexpr Shapes two = {{32, 32 * n, (f32 ? 768 : 384) / (32 * n)}, {8, (8 * n + 31) & ~31, 1}, none, none};
+  constexpr LineShape p1w = f32 ? LineShape{32, 384, 2} : LineShape{16, 192, 2}, p1n = {8, 96, 1};
+  constexpr bool wide1 = !f32 && !VISC;
+  constexpr Shapes p1 = {wide1 ? LineShape{32, 192, 2} : p1w, wide1 ? p1w : p1n, wide1 ? p1n : none, none};
+  constexpr Shapes p2 = {f32 ? LineShape{32, 288, 2} : LineShape{16, 224, 2}, {16, 448, 1}, {8, 224, 1}, none};
+  constexpr LineShape p3n = {4, VISC ? 256 : 192, 1};
+  constexpr Shapes p3 = {f32 ? LineShape{32, 768, 1} : LineShape{16, 384, 1},
+                         f32 ? LineShape{16, 768, 1} : LineShape{8, 384, 1},
+                         VISC && f32 ? LineShape{8, 512, 1} : p3n, VISC && f32 ? p3n : none};
+  constexpr Shapes p4 = {f32 ? LineShape{16, 608, 1} : LineShape{8, VISC ? 608 : 320, 1}, {8, 608, 1},
+                         {4, VISC && f32 ? 512 : 320, 1}, VISC && !f32 ? LineShape{2, 256, 1} : none};
   return C::DIM == 2 ? two[tier] : C::P == 1 ? p1[tier] : C::P == 2 ? p2[tier] : C::P == 3 ? p3[tier] : p4[tier];
 }
 template <class C, typename R, typename S, bool BC, int RS, bool VISC, int TIER = 0>

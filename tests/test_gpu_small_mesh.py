@@ -39,3 +39,37 @@ def test_programmatic_launches_do_not_slow_a_step(monkeypatch, dims, precision):
             s.update(160)
             best[pdl] = min(best.get(pdl, 1.0), time.perf_counter() - t)
     assert best["1"] < 1.2 * best["0"], best
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("order, dims, visc", [
+    (3, (5, 5, 5), 1),     # 32 tiles of 4, the last with one element
+    (4, (5, 5, 5), 1),     # FP64: 63 tiles of 2, the last with one element
+    (4, (7, 7, 6), 1),     # 147 tiles of 2, under one to a multiprocessor
+    (4, (11, 9, 3), 1),    # 297: 75 tiles of 4
+    (1, (23, 17, 17), 0),  # 6647: 208 tiles of 32, the last with 23 elements
+])
+def test_shapes_of_small_viscous_and_first_order_meshes(oracle, order, dims, visc, precision):
+    """State after three steps, and the FP64 residual, against the oracle: 1e-12 in
+    FP64 (rounding), the mixed mode's state 1e-6 in the 2-norm, as every parity test."""
+    from fr_learn_b200 import Solver, box3d
+
+    mesh = box3d(*dims, (0.0,) * 3, (1.0,) * 3, perturb=0.1, seed=3)
+    kw = dict(order=order, **(dict(dtType=0, dt=1e-4, **NS) if visc else dict(dtType=1, CFL=0.4, pBound=1 / 1.4)))
+    oracle.lib().orc_set_threads(16)
+    o = oracle.Oracle(oracle.params(nDims=3, **kw), mesh)
+    g = Solver(mesh, precision=precision, **kw)
+    U = _state(g, 3)
+    o.set("U_spts", U)
+    g.set("U_spts", U)
+    if precision == 0:
+        o.calc_residual(0)
+        g.calcResidual(0)
+        assert relerr(g.get("divF_spts"), o.divF(0)) < 1e-12
+    o.update(3)
+    g.update(3)
+    got, want = g.get("U_spts").ravel(), o.U().ravel()
+    if precision == 0:
+        assert relerr(got, want) < 1e-12
+    else:
+        assert np.linalg.norm(got - want) < 1e-6 * np.linalg.norm(want)
