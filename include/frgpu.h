@@ -289,8 +289,9 @@ frg_status frg_set_stream(frg_solver *s, void *stream);
  * stage k's kernel, all in milliseconds ([1 + nRK] entries). */
 frg_status frg_time_stages(frg_solver *s, int nsteps, void *flush, unsigned long long flushBytes, double *ms_out);
 /* Picks the fastest tile shape (elements x threads per block) of the fused
- * TMA stage kernel for this mesh and configuration by timing `nsteps` steps
- * of each candidate, then restores the solution, time, dt and iteration the
+ * 2D stage kernel for this mesh and configuration by timing `nsteps` steps
+ * of each candidate back to back (the working set as warm in L2 as steps
+ * leave it), then restores the solution, time, dt and iteration the
  * handle had.  Results do not depend on the choice.  `variant_out` receives
  * the chosen index; `ms_out` (may be NULL) one time per step per candidate
  * (frg_tile_variant_count entries, at most FRG_MAX_TILE_VARIANTS).  A no-op
