@@ -1,6 +1,6 @@
 // adjoint_visc.cuh -- vector-Jacobian product of a VISCOUS (LDG) residual
-// evaluation, FP64.  The forward residual (the generic viscous kernels,
-// kernels.cuh) is, per element, with U the stage state:
+// evaluation, FP64.  The forward residual (the viscous line kernels,
+// kernels_line.cuh) is, per element, with U the stage state:
 //
 //   traces     U_f  = sum_j lag[side][j] U[line pt j]
 //   LDG        Dc_f = Uc(U_L, U_R, n) - U_f         (face::ldgSolution)
@@ -16,9 +16,9 @@
 // The transposed chain runs in three element passes after the face-seed
 // pass of the inviscid adjoint (traces of the stage state and this side's
 // share +-dA C^T gbar of the common-flux adjoint):
-//   pass 1  the forward gradient and each side's projected viscous flux (the
-//           generic gradient kernel, fr_visc_grad_kernel), which the
-//           neighbours' face fluxes read as constants;
+//   pass 1  the forward gradient and each side's projected viscous flux
+//           (fr_line_grad_kernel), which the neighbours' face fluxes read as
+//           constants;
 //   pass 2  per flux point, the own-side Jacobian of the common flux
 //           (both elements evaluate the same face flux, each differentiates
 //           with respect to its own trace and gradient trace); per solution

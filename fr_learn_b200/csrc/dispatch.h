@@ -97,7 +97,7 @@ cudaError_t launch_op_gemm(const CUtensorMap &mX, const float *Bimg, float *Y, i
 // reference layout [nS][nE][d].
 struct MetricOut {
   double *pos, *detJd, *nrmOwn, *dAd, *vol;
-  void *JG, *detJs, *invDetS, *nrmC, *dAs;  // stored type (storeBytes)
+  void *JG, *invDetS, *nrmC, *dAs;  // stored type (storeBytes)
 };
 // check != 0: only tests the solution-point Jacobians, flag[0] |= 1 and
 // flag[1] = min element when one is negative; else writes every metric.

@@ -201,11 +201,6 @@ __global__ void __launch_bounds__(128) fr_to_ref_layout(const double *__restrict
   double *r = ref + ((size_t)pt * nE + e) * NV;
   for (int v = 0; v < NV; v++) r[v] = dev[((size_t)v * NPT + pt) * L + e];
 }
-template <typename S>
-__global__ void fr_cast_kernel(const double *in, S *out, long n) {
-  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) out[i] = (S)in[i];
-}
 
 bool select_kernels(const KernelKey &key, KernelSet &k, std::string &err) {
   if (key.nDims == 2) return key.precision == FRG_FP64 ? select_2d_f64(key, k, err) : select_2d_f32(key, k, err);
@@ -237,7 +232,7 @@ struct frg_solver {
   // device buffers
   double *U = nullptr, *U0 = nullptr, *Acc = nullptr, *divF[5] = {nullptr};
   void *W[2] = {nullptr, nullptr}, *tr[2] = {nullptr, nullptr};
-  void *nrm = nullptr, *dAs = nullptr, *JG = nullptr, *detJs = nullptr;
+  void *nrm = nullptr, *dAs = nullptr, *JG = nullptr;
   void *invDetS = nullptr;  // 1 / detJ in the stored type, for the TMA stage kernel
   void *fvn = nullptr, *fvn2 = nullptr;  // viscous: projected viscous flux per flux point
   void *dUg = nullptr;                   // viscous: corrected gradient at the solution points
@@ -642,7 +637,7 @@ int dt_mode(const frg_solver *s) {
 
 // One fused step (the body of solver::update) on the stream.  With `ev`
 // (2 + nRK events) an event is recorded before the dt kernels and after each
-// launch, for frg_time_stages.  With the TMA kernel the last stage computes
+// launch, for frg_time_stages.  The last stage computes
 // the next step's dt (calcDt reads the wave speeds the last stage leaves).
 // `chained`: the previous kernel on the stream is the last stage of the step
 // before, so the first stage too can be its programmatic dependent.
@@ -802,8 +797,7 @@ frg_status frg_create(const frg_params *params, const frg_mesh *mesh, frg_solver
   const int nE = s->nE, L = s->L;
   if ((st = upload_store(s.get(), &s->nrm, pad_rows(s->g.nrmC, nE, L, 0.0))) ||
       (st = upload_store(s.get(), &s->dAs, pad_rows(s->g.dA, nE, L, 0.0))) ||
-      (st = upload_store(s.get(), &s->JG, pad_rows(s->g.JG, nE, L, 0.0))) ||
-      (st = upload_store(s.get(), &s->detJs, pad_rows(s->g.detJ, nE, L, 1.0))))
+      (st = upload_store(s.get(), &s->JG, pad_rows(s->g.JG, nE, L, 0.0))))
     return st;
   {
     std::vector<double> inv = pad_rows(s->g.detJ, nE, L, 1.0);
@@ -921,7 +915,7 @@ frg_status frg_destroy(frg_solver *s) {
   for (double *q : dp) if (q) cudaFree(q);
   cudaFree(s->grpDt);
   cudaFree(s->grpTime);
-  void *vp[] = {s->grp, s->W[0], s->W[1], s->tr[0], s->tr[1], s->nrm, s->dAs, s->JG, s->detJs, s->invDetS, s->nbr, s->err,
+  void *vp[] = {s->grp, s->W[0], s->W[1], s->tr[0], s->tr[1], s->nrm, s->dAs, s->JG, s->invDetS, s->nbr, s->err,
                 s->ticket,
                 s->fvn, s->fvn2, s->dUg};
   for (void *q : vp) if (q) cudaFree(q);
@@ -966,7 +960,7 @@ frg_status frg_update_geometry(frg_solver *s, const double *xv) {
   CK(cudaMemcpyAsync(s->xvDev, xv, nX * 8, cudaMemcpyHostToDevice, s->stream));
   const unsigned init[2] = {0u, 0xffffffffu};
   CK(cudaMemcpyAsync(s->geoFlag, init, sizeof init, cudaMemcpyHostToDevice, s->stream));
-  MetricOut out{s->posDev, s->detJd, s->nrmOwn, s->dAd, s->vol, s->JG, s->detJs, s->invDetS, s->nrm, s->dAs};
+  MetricOut out{s->posDev, s->detJd, s->nrmOwn, s->dAd, s->vol, s->JG, s->invDetS, s->nrm, s->dAs};
   // a negative Jacobian leaves the solver's metrics as they were
   CK(launch_metrics(d, (int)s->sstore, s->xvDev, s->geoTab, fdir, fsgn, wv, s->nbr, nN, nS, nF, nE, L, 1, out,
                     s->geoFlag, s->stream));

@@ -166,14 +166,13 @@ struct StageArgs {
   void *fvnOut, *fvn2Out;
   const void *fvnIn, *fvn2In;
   int visc2;
-  // viscous path, optional: the corrected physical gradient at the solution
-  // points (S), [DIM][NV][NS][nE], written by the gradient kernel and read by
-  // the stage kernel instead of recomputing it (null: recompute)
+  // optional output of the gradient pass: the corrected physical gradient at the
+  // solution points (S), [DIM][NV][NS][nE], for the boundary integrals and the adjoint
   void *dUg;
   // SF_DTNEXT: the next step's dt (ele::calcDt + the global minimum)
   const double *vol, *dAd, *wsurf;
   double *blockMin, *dtNext, *eleDt;
-  // first stage of a step with the fused dt (TMA kernels): the next step's dt
+  // first stage of a step with the fused dt: the next step's dt
   // slot, set here to a huge value before the last stage minimises into it
   double *dtReset;
   unsigned *ticket;

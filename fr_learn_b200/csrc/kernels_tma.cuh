@@ -1,8 +1,8 @@
 // kernels_tma.cuh -- the RK stage kernel of the fused update path with its
 // tiles moved by the Tensor Memory Accelerator.
 //
-// The generic stage kernel (kernels.cuh) loads its inputs with per-thread
-// loads, so each phase waits on a few loads in flight per thread.  Here one
+// The line kernels (kernels_line.cuh) load their inputs with per-thread loads, so
+// each phase waits on the loads in flight per thread.  Here one
 // thread issues, at block start, every tile the block will need as 2D bulk
 // tensor copies (cp.async.bulk.tensor) into shared memory, in three groups
 // completing on three mbarriers:

@@ -95,7 +95,6 @@ __global__ void __launch_bounds__(256) fr_metrics_kernel(const double *__restric
     }
     const size_t q = (size_t)s * L + e;
     out.detJd[q] = det;
-    put<S>(out.detJs, q, det);
     put<S>(out.invDetS, q, __ddiv_rn(1.0, det));
 #pragma unroll
     for (int a = 0; a < D; a++)
